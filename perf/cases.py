@@ -235,7 +235,8 @@ def _prepare_host(case, make):
         a_at += m * k
         d_at += m * n
     batch = _capi.HostBatch(calls, torch.device("cuda", torch.cuda.current_device()))
-    return {"kind": "host", "batch": batch, "stream": torch.cuda.Stream(), "outputs": [c[2] for c in calls]}
+    return {"kind": "host", "batch": batch, "stream": torch.cuda.Stream(), "outputs": [c[2] for c in calls],
+            "keep": calls}
 
 
 def prepare(case, seed):
@@ -332,3 +333,76 @@ def tolerance(case):
         return {"rel": 5e-4, "max": 0.15}
     # several roundings to bf16 and fp8 in a row: up to 2.6e-3, largest single difference 5e-2
     return {"rel": 1e-2, "max": 0.15}
+
+
+# ------------------------------------------------------------------------------- 64-bit results
+def _matmul(a, w_nk, scale, bias=None):
+    """scale * (a @ w^T) + bias in float64, a block of weight rows at a time."""
+    a64, out = a.double(), []
+    for rows in w_nk.cuda().split(8192):
+        out.append(a64 @ rows.double().t())
+    result = torch.cat(out, dim=1) * scale.double()
+    return result if bias is None else result + bias.double()
+
+
+def _quantise(y, fp8):
+    """What an fp8 buffer holds of y; both formats saturate at the largest finite e4m3fn byte."""
+    top = 224.0 if fp8 == torch.float8_e4m3fnuz else 448.0
+    return y.clamp(-top, top), y.clamp(-top, top).float().to(fp8)
+
+
+def _norm64(x, residual, weight):
+    """The 16-bit sum that the norm reads, the sum before that rounding, the normalised rows."""
+    exact_sum = x.double() + residual.double()
+    s = exact_sum.to(x.dtype).double()
+    return exact_sum, s * torch.rsqrt(s.square().mean(dim=1, keepdim=True) + _EPS) * weight.double()
+
+
+def _swiglu64(gate_up, scale):
+    gate, up = gate_up.double().chunk(2, dim=1)
+    return torch.nn.functional.silu(gate) * up / scale.double()
+
+
+def _mlp64(x, residual, w):
+    fp8 = w["gate_up_weight"].dtype
+    new_residual, y = _norm64(x, residual, w["rms_weight"])
+    normed = _quantise(y / w["gate_up_input_scale"].double(), fp8)[1]
+    gate_up = _matmul(normed, w["gate_up_weight"].t(), w["gate_up_output_scale"]).to(x.dtype)
+    act = _quantise(_swiglu64(gate_up, w["down_input_scale"]), fp8)[1]
+    return _matmul(act, w["down_weight"].t(), w["down_output_scale"]), new_residual
+
+
+def exact(case, seed):
+    """The outputs of ``run`` from torch in float64. Values that the operators hand on in 16 or 8 bits are
+    rounded to them in between, as the operators define it; the returned ones are not rounded."""
+    state = prepare(case, seed)
+    kind = case["kind"]
+    if kind == "gemm":
+        return _matmul(state["a"], state["b"].t(), state["scale"], state["bias"])
+    if kind == "mlp":
+        return _mlp64(state["x"], state["residual"], state["weights"])
+    if kind == "rms":
+        new_residual, y = _norm64(state["x"], state["residual"], state["weight"])
+        if state["scale"] is None:
+            return y, new_residual
+        y = _quantise(y / state["scale"].double(), state["fp8"])[0]
+        return (y, new_residual) if state["buffer"] is None else (y, new_residual, torch.zeros_like(state["buffer"]))
+    if kind == "swiglu":
+        y = _quantise(_swiglu64(state["gate_up"], state["scale"]), state["fp8"])[0]
+        return y if state["buffer"] is None else (y, torch.zeros_like(state["buffer"]))
+    if kind == "host":
+        results = []
+        for call in state["keep"]:
+            bias = call[5].cuda() if len(call) > 5 else None
+            results.append(_matmul(call[0].cuda(), call[1], call[3], bias))
+        return results
+    layers, hidden_in, residual_in = state["keep"]
+    results = []
+    for w, x, residual in zip(layers, hidden_in, residual_in):
+        new_residual, y = _norm64(x, residual, w["norm"])
+        normed = _quantise(y / w["norm_scale"].double(), w["w_qkv"].dtype)[1]
+        o_out = _matmul(w["attn_out"], w["w_o"].t(), w["o_scale"]).to(x.dtype)
+        hidden, new_residual = _mlp64(o_out, new_residual.to(x.dtype), w["mlp"])
+        results.append({"qkv": _matmul(normed, w["w_qkv"].t(), w["qkv_scale"]), "hidden": hidden,
+                        "residual": new_residual})
+    return results
