@@ -45,6 +45,7 @@
 #include "device_model.cuh"
 #include "skinny_gemm_kernel.cuh"
 #include "skinny_gemm_streamk.cuh"
+#include "skinny_gemm_wide.cuh"
 
 namespace hfrk {
 
@@ -410,6 +411,11 @@ int prepare_device_once() {
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
     HFRK_CUDA_TRY(cudaFuncSetAttribute(skinny_gemm_fp8_streamk_kernel<2>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
+    for (const void* fn : {reinterpret_cast<const void*>(skinny_gemm_fp8_wide_kernel<false>),
+                           reinterpret_cast<const void*>(skinny_gemm_fp8_wide_kernel<true>)}) {
+        HFRK_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
+        HFRK_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    }
     if (dev >= 0 && dev < 64) done[dev] = true;
     return HFRK_SUCCESS;
 }
@@ -590,6 +596,209 @@ int launch_streamk(const void* A, const void* W, void* D, const float* scale_dev
     return HFRK_SUCCESS;
 }
 
+// ---------------------------------------------------------------- wide kernel (65 .. 256 tokens per launch)
+struct WidePlan {
+    int halves, rows_half, tile_n, tiles, split, stages, acc_cols, tmem_cols, num_kblocks, smem_bytes;
+};
+
+struct WideReq {
+    int split = 0, tile_n = 0, stages = 0, per_sm = 0;   // 0 = choose
+};
+
+// Estimated time of one launch in microseconds. The stream of K blocks runs at the slowest of: W out of
+// HBM, all loads out of L2, the loads of the busiest SM, the tensor core of the busiest SM, and the
+// latency of a load over the stages that hide it. To it come the fixed cost of a call in a chain of
+// dependent calls, one per further wave, the epilogue's stores and, with a K split, the cluster barrier
+// and the partials that a CTA sends to its peers (~40 GB/s per SM). The constants are a fit to
+// 3,900 timings on a B200 (114 shapes of 17 to 256 tokens, every tile height, split and CTAs per SM that
+// fits): the shape it picks is on average 4.5 % slower than the best of its list, 26 % at worst.
+struct WideCost {
+    int n, k, halves, rows, tile_n, split, stages, per_sm, ctas, waves, ctas_busiest, kb;
+};
+
+double wide_cost_us(const WideCost& c) {
+    const double bytes_kb = static_cast<double>(c.rows + c.tile_n) * kBlockK;
+    double t = static_cast<double>(c.n) * c.k / 8.02e6;
+    const auto at_least = [&t](double v) { t = v > t ? v : t; };
+    at_least(static_cast<double>(c.ctas) * c.kb * bytes_kb / 9.07e6);
+    at_least(static_cast<double>(c.ctas_busiest) * c.kb * bytes_kb / 7.37e4);
+    at_least(static_cast<double>(c.ctas_busiest) * c.kb * c.halves * c.tile_n * (1.67 * 2.0 / 1900.0));
+    at_least(c.waves * c.kb * 1.06 / (c.stages > 2 ? c.stages - 1 : 1));
+    const double outputs = static_cast<double>(c.ctas_busiest) * c.rows * c.tile_n;   // of the busiest SM
+    t += 4.12 + (c.waves - 1) * 4.48 + 1.9e-7 * outputs / c.split;
+    if (c.split > 1) t += 0.353 + 2.43e-5 * outputs * 4.0 * (c.split - 1) / c.split;
+    if (c.per_sm == 2 && c.waves == 1) t -= 0.344;   // CTAs of the next call move in earlier
+    return t;
+}
+
+int search_wide_plan(const DeviceModel& dm, int m, int n, int k, bool swiglu, const WideReq& req, WidePlan* plan) {
+    if (m <= 0 || n <= 0 || k <= 0 || m > kWideMaxTokens) return HFRK_INVALID_CONFIG;
+    const int halves = m > 128 ? 2 : 1;
+    const int rows_half = round_up((m + halves - 1) / halves, 8);
+    const int nkb = (k + kBlockK - 1) / kBlockK;
+    const int step = swiglu ? 32 : 16;
+    double best = 0.0;
+    bool found = false;
+    for (int split = 1; split <= kWideMaxSplit && split <= nkb; ++split) {
+        if (req.split != 0 && split != req.split) continue;
+        for (int tile_n = 32; tile_n <= kWideMaxTile; tile_n += step) {
+            if (req.tile_n != 0 && tile_n != req.tile_n) continue;
+            const int groups = tile_n / step;
+            if (groups < split) continue;   // every CTA of a cluster finishes something
+            const int tiles = (n + tile_n - 1) / tile_n;
+            int acc_cols = 32;
+            while (acc_cols < tile_n) acc_cols *= 2;
+            const int tmem_cols = halves * acc_cols;
+            const int stage_bytes = halves * kWideSlotBytes + tile_n * kBlockK;
+            const int recv_bytes = split > 1 ? split * ((groups + split - 1) / split) * step * (halves * rows_half + 1) * 4
+                                             : kWideTurnBytes;
+            for (int per_sm = 1; per_sm <= 2; ++per_sm) {
+                if (req.per_sm != 0 && per_sm != req.per_sm) continue;
+                const int budget = kSmemPerSm / per_sm - kSmemCtaReserve;
+                const int limit = budget < kSmemLimit ? budget : kSmemLimit;
+                int stages = (limit - 1024 - kCtrlBytes) / stage_bytes;
+                if (stages > kWideMaxStages) stages = kWideMaxStages;
+                if (req.stages != 0 && stages > req.stages) stages = req.stages;
+                if (stages < 2 || tmem_cols * per_sm > 512) continue;
+                if (recv_bytes > stages * stage_bytes) continue;
+                if (split > 1 && tiles > dm.capacity[split][per_sm]) continue;
+                int smem = 1024 + stages * stage_bytes + kCtrlBytes;
+                // CTAs that share an SM must never ask for more TMEM than it has: a CTA that waits for
+                // columns keeps its cluster waiting. Every kernel's share of the shared memory is at least its
+                // share of the 512 columns, so what fits in shared memory fits in TMEM.
+                const int smem_floor = kSmemPerSm / 512 * tmem_cols - kSmemCtaReserve;
+                if (smem < smem_floor) smem = smem_floor;
+                if (smem > kSmemLimit) continue;
+
+                const int ctas = tiles * split;
+                const int slots = dm.sms * per_sm;
+                const int waves = (ctas + slots - 1) / slots;
+                const int ctas_busiest = waves == 1 ? (ctas + dm.sms - 1) / dm.sms : waves * per_sm;
+                const WideCost c{n, k, halves, halves * rows_half, tile_n, split, stages, per_sm, ctas, waves, ctas_busiest,
+                                 (nkb + split - 1) / split};
+                const double t = wide_cost_us(c);
+                if (!found || t < best) {
+                    found = true;
+                    best = t;
+                    *plan = WidePlan{halves, rows_half, tile_n, tiles, split, stages, acc_cols, tmem_cols, nkb, smem};
+                }
+            }
+        }
+    }
+    return found ? HFRK_SUCCESS : HFRK_INVALID_CONFIG;
+}
+
+// The search costs some 5 us of host time, as much as the rest of an eager call. Each thread keeps the
+// plans of its last shapes (a fixed table, one slot per hash), with the device model they were made for.
+int make_wide_plan(const DeviceModel& dm, int m, int n, int k, bool swiglu, const WideReq& req, WidePlan* plan) {
+    struct Slot {
+        int m = 0, n = 0, k = 0;
+        bool swiglu = false;
+        WideReq req;
+        DeviceModel dm;
+        WidePlan plan;
+    };
+    constexpr unsigned kSlots = 64;
+    static thread_local Slot slots[kSlots];
+    const unsigned hash = static_cast<unsigned>(m) * 40503u ^ static_cast<unsigned>(n) * 2654435761u ^
+                          static_cast<unsigned>(k) * 2246822519u ^ (swiglu ? 0x9E3779B9u : 0u);
+    Slot& slot = slots[(hash ^ (hash >> 16)) % kSlots];
+    if (slot.m == m && slot.n == n && slot.k == k && slot.swiglu == swiglu && slot.dm.sms == dm.sms &&
+        memcmp(&slot.req, &req, sizeof(req)) == 0 && memcmp(slot.dm.capacity, dm.capacity, sizeof(dm.capacity)) == 0) {
+        *plan = slot.plan;
+        return HFRK_SUCCESS;
+    }
+    const int rc = search_wide_plan(dm, m, n, k, swiglu, req, plan);
+    if (rc == HFRK_SUCCESS) slot = Slot{m, n, k, swiglu, req, dm, *plan};
+    return rc;
+}
+
+// Which calls the wide kernel takes, unless the caller (or the tuning table) asked for a launch shape of
+// the skinny kernel:
+//   * more tokens than one launch of the skinny kernel holds: 28672 x 4096 at 256 tokens 31 us against 91;
+//   * 17 to 64 tokens where the skinny kernel's unsplit grid needs a second wave, because its activation
+//     tile leaves room for two CTAs per SM: 39840 x 6272 at 30 tokens 42 us against 55. In one wave the
+//     two are within a few percent of each other, and up to 16 tokens the skinny kernel is always ahead.
+bool use_wide_kernel(const DeviceModel& dm, int m, int n, int k, bool explicit_shape) {
+    if (explicit_shape || m <= 16) return false;
+    TuneValue tuned;
+    const int mc = m < kMaxMPad ? m : kMaxMPad;
+    if (tuning_lookup(round_up(mc, 16), n, k, &tuned)) return false;
+    if (m > kMaxMPad) return true;
+    Plan plan;
+    if (make_plan(dm, m, n, k, 0, 0, &plan) != HFRK_SUCCESS) return false;
+    return plan.split == 1 && plan.ctas > ctas_per_sm(plan.smem_bytes) * dm.sms;
+}
+
+// One launch per 256 tokens, the tokens shared out evenly. The caller has validated the arguments.
+// `p` carries the outputs (d or act_out / zero_ptr of the whole call) and the scalars.
+template <bool kSwiglu>
+int launch_wide(const void* A, const void* W, int m, int n, int k, int64_t w_row_stride, WideParams p, int use_pdl,
+                cudaStream_t stream) {
+    const DeviceModel dm = device_model(stream);
+    const int chunks = (m + kWideMaxTokens - 1) / kWideMaxTokens;
+    const int m_step = (m + chunks - 1) / chunks;
+    uint8_t* const d = static_cast<uint8_t*>(p.d);
+    uint8_t* const act_out = p.act_out;
+    const size_t out_elem = p.d_dtype == HFRK_F32 ? 4 : 2;
+    for (int m0 = 0; m0 < m; m0 += m_step) {
+        const int mc = m - m0 < m_step ? m - m0 : m_step;
+        WidePlan plan;
+        const WideReq req;
+        int rc = make_wide_plan(dm, mc, n, k, kSwiglu, req, &plan);
+        if (rc != HFRK_SUCCESS) return rc;
+        const int tile_rows = kSwiglu ? plan.tile_n / 2 : plan.tile_n;
+        CUtensorMap tmap_w, tmap_a;
+        rc = get_tensor_map(W, static_cast<uint64_t>(k), static_cast<uint64_t>(n), static_cast<uint64_t>(w_row_stride),
+                            static_cast<uint32_t>(tile_rows), &tmap_w);
+        if (rc != HFRK_SUCCESS) return rc;
+        rc = get_tensor_map(static_cast<const uint8_t*>(A) + static_cast<size_t>(m0) * k, static_cast<uint64_t>(k),
+                            static_cast<uint64_t>(mc), static_cast<uint64_t>(k), static_cast<uint32_t>(plan.rows_half),
+                            &tmap_a);
+        if (rc != HFRK_SUCCESS) return rc;
+        p.m = mc;
+        p.n = n;
+        p.halves = plan.halves;
+        p.rows_half = plan.rows_half;
+        p.tile_n = plan.tile_n;
+        p.acc_cols = plan.acc_cols;
+        p.tmem_cols = plan.tmem_cols;
+        p.num_kblocks = plan.num_kblocks;
+        p.split = plan.split;
+        p.stages = plan.stages;
+        if (kSwiglu) {
+            p.act_out = act_out + static_cast<size_t>(m0) * p.act_cols;
+            if (m0 > 0) p.zero_bytes = 0;   // the first launch clears the whole buffer
+        } else {
+            p.d = d + static_cast<size_t>(m0) * n * out_elem;
+        }
+        cudaLaunchConfig_t cfg = {};
+        const int tiles = kSwiglu ? (p.act_cols + tile_rows - 1) / tile_rows : plan.tiles;
+        cfg.gridDim = dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(plan.split), 1);
+        cfg.blockDim = dim3(kWideThreads, 1, 1);
+        cfg.dynamicSmemBytes = static_cast<size_t>(plan.smem_bytes);
+        cfg.stream = stream;
+        cudaLaunchAttribute attrs[2];
+        unsigned num_attrs = 0;
+        if (plan.split > 1) {
+            attrs[num_attrs].id = cudaLaunchAttributeClusterDimension;
+            attrs[num_attrs].val.clusterDim.x = 1;
+            attrs[num_attrs].val.clusterDim.y = static_cast<unsigned>(plan.split);
+            attrs[num_attrs].val.clusterDim.z = 1;
+            ++num_attrs;
+        }
+        if (use_pdl) {
+            attrs[num_attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attrs[num_attrs].val.programmaticStreamSerializationAllowed = 1;
+            ++num_attrs;
+        }
+        cfg.attrs = attrs;
+        cfg.numAttrs = num_attrs;
+        HFRK_CUDA_TRY(cudaLaunchKernelEx(&cfg, skinny_gemm_fp8_wide_kernel<kSwiglu>, tmap_w, tmap_a, p));
+    }
+    return HFRK_SUCCESS;
+}
+
 int launch_gemm(const void* A, const void* W, void* D, const float* scale_dev, int m, int n, int k,
                 int64_t w_row_stride, int a_kind, int w_kind, int d_dtype, int accumulate, int variant,
                 int split_req, int ctas_per_sm, int stages_req, int use_pdl, cudaStream_t stream,
@@ -600,11 +809,24 @@ int launch_gemm(const void* A, const void* W, void* D, const float* scale_dev, i
     rc = prepare_device_once();
     if (rc != HFRK_SUCCESS) return rc;
     if (variant < HFRK_VARIANT_AUTO || variant > HFRK_VARIANT_STREAMK) return HFRK_INVALID_CONFIG;
+    const bool explicit_shape = variant != HFRK_VARIANT_AUTO || split_req != 0 || ctas_per_sm != 0 || stages_req != 0 ||
+                                tile_rows_req != 0 || stamps != nullptr;
     if (variant == HFRK_VARIANT_AUTO) variant = HFRK_VARIANT_CLUSTER;
     if (rowpar != nullptr && variant != HFRK_VARIANT_CLUSTER) return HFRK_INVALID_CONFIG;
     if (variant == HFRK_VARIANT_STREAMK) {
         return launch_streamk(A, W, D, scale_dev, m, n, k, w_row_stride, a_kind, w_kind, d_dtype, accumulate,
                               ctas_per_sm, stages_req, use_pdl, stream, stamps);
+    }
+
+    if (use_wide_kernel(device_model(stream), m, n, k, rowpar != nullptr || explicit_shape)) {
+        WideParams p;
+        memset(&p, 0, sizeof(p));
+        p.d = D;
+        p.scale = scale_dev;
+        p.kind_factor = (a_kind == HFRK_E4M3FNUZ ? 0.5f : 1.0f) * (w_kind == HFRK_E4M3FNUZ ? 0.5f : 1.0f);
+        p.d_dtype = d_dtype;
+        p.accumulate = accumulate ? 1 : 0;
+        return launch_wide<false>(A, W, m, n, k, w_row_stride, p, use_pdl, stream);
     }
 
     const size_t out_elem = d_dtype == HFRK_F32 ? 4 : 2;
@@ -697,14 +919,16 @@ int launch_gemm(const void* A, const void* W, void* D, const float* scale_dev, i
 // grid takes gate rows [64t, 64t + 64) and up rows [inter + 64t, inter + 64t + 64), so that both
 // halves of every output column meet in one CTA. With a K split the cluster's reduction hands every
 // CTA whole token rows of the tile (not arbitrary element ranges), so the halves still meet.
+// More than 16 tokens: the same chain element in the wide kernel (launch_wide<true>), in launches of up
+// to 256 tokens.
 int launch_gemm_swiglu(const void* A, const void* W, void* act_out, const float* scale_dev,
                        const float* act_scale_dev, void* next_buffer, int m, int inter, int k, int64_t w_row_stride,
                        int a_kind, int w_kind, int mid_dtype, int out_kind, int64_t buffer_cols, int split_req,
-                       int use_pdl, cudaStream_t stream) {
+                       int use_pdl, bool any_tokens, cudaStream_t stream) {
     if (A == nullptr || W == nullptr || act_out == nullptr || scale_dev == nullptr || act_scale_dev == nullptr)
         return HFRK_INVALID_CONFIG;
     if (m <= 0 || inter <= 0 || k <= 0 || buffer_cols < 0) return HFRK_INVALID_CONFIG;
-    if (m > 16) return HFRK_TOO_LARGE;
+    if (m > 16 && !any_tokens) return HFRK_TOO_LARGE;
     if (inter % 16 != 0) return HFRK_INVALID_CONFIG;   // 16-byte pieces of the fp8 output rows
     if ((a_kind != HFRK_E4M3FN && a_kind != HFRK_E4M3FNUZ) || (w_kind != HFRK_E4M3FN && w_kind != HFRK_E4M3FNUZ) ||
         (mid_dtype != HFRK_F16 && mid_dtype != HFRK_BF16) || (out_kind != HFRK_E4M3FN && out_kind != HFRK_E4M3FNUZ))
@@ -718,6 +942,22 @@ int launch_gemm_swiglu(const void* A, const void* W, void* act_out, const float*
         return HFRK_BAD_ALIGNMENT;
     int rc = prepare_device_once();
     if (rc != HFRK_SUCCESS) return rc;
+
+    if (m > 16) {
+        if (inter > INT32_MAX / 2) return HFRK_INVALID_CONFIG;
+        WideParams wp;
+        memset(&wp, 0, sizeof(wp));
+        wp.scale = scale_dev;
+        wp.kind_factor = (a_kind == HFRK_E4M3FNUZ ? 0.5f : 1.0f) * (w_kind == HFRK_E4M3FNUZ ? 0.5f : 1.0f);
+        wp.d_dtype = mid_dtype;
+        wp.act_out = static_cast<uint8_t*>(act_out);
+        wp.act_scale = act_scale_dev;
+        wp.act_cols = inter;
+        wp.act_fnuz = out_kind == HFRK_E4M3FNUZ ? 1 : 0;
+        wp.zero_ptr = static_cast<uint8_t*>(next_buffer);
+        wp.zero_bytes = zero_bytes;
+        return launch_wide<true>(A, W, m, 2 * inter, k, w_row_stride, wp, use_pdl, stream);
+    }
 
     CUtensorMap tmap_w, tmap_a;
     rc = get_tensor_map(W, static_cast<uint64_t>(k), static_cast<uint64_t>(2) * inter,
@@ -1057,7 +1297,16 @@ extern "C" int hfrk_skinny_gemm_fp8_swiglu(const void* A, const void* W_gate_up,
                                            int mid_dtype, int out_kind, int64_t buffer_cols, void* stream) {
     return hfrk::launch_gemm_swiglu(A, W_gate_up, act_out, scale_dev, act_scale_dev, next_buffer, m, inter, k,
                                     w_row_stride, a_kind, w_kind, mid_dtype, out_kind, buffer_cols, /*split_req=*/0,
-                                    hfrk::default_use_pdl(), static_cast<cudaStream_t>(stream));
+                                    hfrk::default_use_pdl(), /*any_tokens=*/false, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int hfrk_gate_up_swiglu_fp8(const void* A, const void* W_gate_up, void* act_out, const float* scale_dev,
+                                       const float* act_scale_dev, void* next_buffer, int m, int inter, int k,
+                                       int64_t w_row_stride, int a_kind, int w_kind, int mid_dtype, int out_kind,
+                                       int64_t buffer_cols, void* stream) {
+    return hfrk::launch_gemm_swiglu(A, W_gate_up, act_out, scale_dev, act_scale_dev, next_buffer, m, inter, k,
+                                    w_row_stride, a_kind, w_kind, mid_dtype, out_kind, buffer_cols, /*split_req=*/0,
+                                    hfrk::default_use_pdl(), /*any_tokens=*/true, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int hfrk_skinny_gemm_fp8_ex(const void* A, const void* W, void* D, const float* scale_dev, int m, int n,

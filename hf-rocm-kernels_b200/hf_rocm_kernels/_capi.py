@@ -34,7 +34,7 @@ EXPORTED_SYMBOLS = (
     "hfrk_rowpar_local_block", "hfrk_rowpar_destroy", "hfrk_skinny_gemm_fp8_rowpar",
     "hfrk_skinny_gemm_fp8_noalloc", "hfrk_max_active_clusters", "hfrk_tuning_set", "hfrk_tuning_clear",
     "hfrk_swiglu_fp8", "hfrk_residual_rms", "hfrk_rowpar_set_mode",
-    "hfrk_skinny_gemm_fp8_swiglu", "hfrk_skinny_gemm_fp8_host_async",
+    "hfrk_skinny_gemm_fp8_swiglu", "hfrk_gate_up_swiglu_fp8", "hfrk_skinny_gemm_fp8_host_async",
     "hfrk_tuning_set_ex", "hfrk_rowpar_set_wait_ms", "hfrk_device_model_get", "hfrk_device_model_override",
 )
 
@@ -101,6 +101,8 @@ def _load() -> ctypes.CDLL:
     lib.hfrk_residual_rms.restype = i32
     lib.hfrk_skinny_gemm_fp8_swiglu.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, i32, i64, i32, i32, i32, i32, i64, vp]
     lib.hfrk_skinny_gemm_fp8_swiglu.restype = i32
+    lib.hfrk_gate_up_swiglu_fp8.argtypes = lib.hfrk_skinny_gemm_fp8_swiglu.argtypes
+    lib.hfrk_gate_up_swiglu_fp8.restype = i32
     lib.hfrk_last_error.restype = ctypes.c_char_p
     for name in ("hfrk_skinny_gemm_fp8", "hfrk_skinny_gemm_fp8_ex", "hfrk_skinny_gemm_fp8_host",
                  "hfrk_skinny_gemm_fp8_simt", "hfrk_skinny_gemm_plan", "hfrk_device_status", "hfrk_version"):

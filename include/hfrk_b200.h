@@ -311,6 +311,16 @@ int hfrk_skinny_gemm_fp8_swiglu(const void* A, const void* W_gate_up, void* act_
                                 int m, int inter, int k, int64_t w_row_stride, int a_kind, int w_kind,
                                 int mid_dtype, int out_kind, int64_t buffer_cols, void* stream);
 
+/* The same operation for any number of tokens, same arguments. Up to 16 tokens it is
+ * hfrk_skinny_gemm_fp8_swiglu; above, launches of up to 256 tokens with the tokens on the tensor
+ * core's M side. The projection may then be summed in another order than by hfrk_skinny_gemm_fp8, so
+ * the bytes agree with the unfused chain up to the rounding of the 16-bit projection.
+ * No counterpart in the reference (see above). */
+int hfrk_gate_up_swiglu_fp8(const void* A, const void* W_gate_up, void* act_out,
+                            const float* scale_dev, const float* act_scale_dev, void* next_buffer,
+                            int m, int inter, int k, int64_t w_row_stride, int a_kind, int w_kind,
+                            int mid_dtype, int out_kind, int64_t buffer_cols, void* stream);
+
 /* Pins the launch shape of (m, n, k) for every later automatic call in this process: split_k and
  * num_stages as in hfrk_skinny_gemm_fp8_ex (0 = leave that one to the built-in rule; both 0 = drop
  * the entry). Token counts share an entry per multiple of 16. Fed from the JSON the grid search
