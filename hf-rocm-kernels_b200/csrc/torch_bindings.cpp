@@ -34,11 +34,8 @@ int out_kind_of(const torch::Tensor& t) {
 // (D += scale * A.B); scale_tensor one fp32 on the device. split_k > 0 requests that K split,
 // 0 lets the library choose; the other eight integers belonged to the reference's MI300X kernel
 // and are ignored.
-int64_t skinny_gemm_tb(torch::Tensor& A, torch::Tensor& B, torch::Tensor& D, torch::Tensor& scale_tensor,
-                       int64_t split_k, int64_t A_producers, int64_t B_producers, int64_t consumers,
-                       int64_t a_lanes, int64_t b_lanes, int64_t qsize, int64_t op_m, int64_t ops) {
-    (void)A_producers; (void)B_producers; (void)consumers; (void)a_lanes;
-    (void)b_lanes; (void)qsize; (void)op_m; (void)ops;
+static int64_t call_skinny_gemm(torch::Tensor& A, torch::Tensor& B, torch::Tensor& D, torch::Tensor& scale_tensor,
+                                int64_t split_k, int accumulate) {
     if (A.dim() != 2 || B.dim() != 2 || B.stride(0) != 1 || !A.is_contiguous() || !D.is_contiguous() ||
         A.size(1) != B.size(0) || D.numel() != A.size(0) * B.size(1) || scale_tensor.numel() != 1 ||
         scale_tensor.scalar_type() != at::ScalarType::Float) {
@@ -55,7 +52,27 @@ int64_t skinny_gemm_tb(torch::Tensor& A, torch::Tensor& B, torch::Tensor& D, tor
     return hfrk_skinny_gemm_fp8(A.data_ptr(), B.data_ptr(), D.data_ptr(),
                                 static_cast<const float*>(scale_tensor.data_ptr()), static_cast<int>(m),
                                 static_cast<int>(n), static_cast<int>(k), B.stride(1), a_kind, w_kind, d_kind,
-                                /*accumulate=*/1, static_cast<int>(split_k > 16 ? 16 : split_k), stream);
+                                accumulate, static_cast<int>(split_k > 16 ? 16 : split_k), stream);
+}
+
+int64_t skinny_gemm_tb(torch::Tensor& A, torch::Tensor& B, torch::Tensor& D, torch::Tensor& scale_tensor,
+                       int64_t split_k, int64_t A_producers, int64_t B_producers, int64_t consumers,
+                       int64_t a_lanes, int64_t b_lanes, int64_t qsize, int64_t op_m, int64_t ops) {
+    (void)A_producers; (void)B_producers; (void)consumers; (void)a_lanes;
+    (void)b_lanes; (void)qsize; (void)op_m; (void)ops;
+    return call_skinny_gemm(A, B, D, scale_tensor, split_k, /*accumulate=*/1);
+}
+
+// The same GEMM into a buffer that holds nothing yet, D = scale * A.B: callers that would only zero D
+// first save that launch, and the kernel does not read D. No counterpart in the reference.
+int64_t skinny_gemm_store(torch::Tensor& A, torch::Tensor& B, torch::Tensor& D, torch::Tensor& scale_tensor) {
+    return call_skinny_gemm(A, B, D, scale_tensor, /*split_k=*/0, /*accumulate=*/0);
+}
+
+// For graph tracers, as skinny_gemm_inplace below.
+void skinny_gemm_store_inplace(torch::Tensor& A, torch::Tensor& B, torch::Tensor& D, torch::Tensor& scale_tensor) {
+    const int64_t status = skinny_gemm_store(A, B, D, scale_tensor);
+    TORCH_CHECK(status == HFRK_SUCCESS, "skinny_gemm: status ", status, " (see hfrk_b200.h)");
 }
 
 // The same GEMM for graph tracers: an op that returns an int cannot be captured into a traced graph,
@@ -66,12 +83,11 @@ void skinny_gemm_inplace(torch::Tensor& A, torch::Tensor& B, torch::Tensor& D, t
     TORCH_CHECK(status == HFRK_SUCCESS, "skinny_gemm: status ", status, " (see hfrk_b200.h)");
 }
 
-// Gate/up projection with swiglu in its epilogue (hfrk_skinny_gemm_fp8_swiglu): A [m, k] fp8, B the
-// [k, 2*inter] view (stride(0) == 1) of the row-major gate/up weight, act_out [m, inter] fp8,
-// next_buffer [m, any] 16-bit zeroed. mid_bf16 names the 16-bit type the unfused chain would have
-// stored the projection in. No counterpart in the reference.
-void skinny_gemm_swiglu(torch::Tensor& A, torch::Tensor& B, torch::Tensor& act_out, torch::Tensor& scale_tensor,
-                        torch::Tensor& act_scale_tensor, torch::Tensor& next_buffer, bool mid_bf16) {
+using GateUpEntry = decltype(&hfrk_skinny_gemm_fp8_swiglu);
+
+static void call_gate_up_swiglu(GateUpEntry entry, torch::Tensor& A, torch::Tensor& B, torch::Tensor& act_out,
+                                torch::Tensor& scale_tensor, torch::Tensor& act_scale_tensor, torch::Tensor& next_buffer,
+                                bool mid_bf16) {
     TORCH_CHECK(A.dim() == 2 && B.dim() == 2 && B.stride(0) == 1 && A.is_contiguous() && act_out.is_contiguous() &&
                     A.size(1) == B.size(0) && B.size(1) % 2 == 0 && act_out.numel() == A.size(0) * (B.size(1) / 2),
                 "skinny_gemm_swiglu: expected A [m, k], B [k, 2*inter] column-major, act_out [m, inter]");
@@ -88,12 +104,27 @@ void skinny_gemm_swiglu(torch::Tensor& A, torch::Tensor& B, torch::Tensor& act_o
     TORCH_CHECK(m <= INT32_MAX && inter <= INT32_MAX && k <= INT32_MAX, "skinny_gemm_swiglu: extent above 2^31");
     const at::cuda::OptionalCUDAGuard device_guard(device_of(A));
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
-    const int status = hfrk_skinny_gemm_fp8_swiglu(
+    const int status = entry(
         A.data_ptr(), B.data_ptr(), act_out.data_ptr(), static_cast<const float*>(scale_tensor.data_ptr()),
         static_cast<const float*>(act_scale_tensor.data_ptr()), next_buffer.data_ptr(), static_cast<int>(m),
         static_cast<int>(inter), static_cast<int>(k), B.stride(1), a_kind, w_kind, mid_bf16 ? HFRK_BF16 : HFRK_F16,
         out_kind, m == 0 ? 0 : next_buffer.numel() / m, stream);
     TORCH_CHECK(status == HFRK_SUCCESS, "skinny_gemm_swiglu: status ", status, " (", hfrk_last_error(), ")");
+}
+
+// Gate/up projection with swiglu in its epilogue (hfrk_skinny_gemm_fp8_swiglu): A [m, k] fp8, B the
+// [k, 2*inter] view (stride(0) == 1) of the row-major gate/up weight, act_out [m, inter] fp8,
+// next_buffer [m, any] 16-bit zeroed. mid_bf16 names the 16-bit type the unfused chain would have
+// stored the projection in. No counterpart in the reference.
+void skinny_gemm_swiglu(torch::Tensor& A, torch::Tensor& B, torch::Tensor& act_out, torch::Tensor& scale_tensor,
+                        torch::Tensor& act_scale_tensor, torch::Tensor& next_buffer, bool mid_bf16) {
+    call_gate_up_swiglu(hfrk_skinny_gemm_fp8_swiglu, A, B, act_out, scale_tensor, act_scale_tensor, next_buffer, mid_bf16);
+}
+
+// The same for any number of tokens (hfrk_gate_up_swiglu_fp8).
+void gate_up_swiglu(torch::Tensor& A, torch::Tensor& B, torch::Tensor& act_out, torch::Tensor& scale_tensor,
+                    torch::Tensor& act_scale_tensor, torch::Tensor& next_buffer, bool mid_bf16) {
+    call_gate_up_swiglu(hfrk_gate_up_swiglu_fp8, A, B, act_out, scale_tensor, act_scale_tensor, next_buffer, mid_bf16);
 }
 
 // gate_up [rows, 2*hidden] fp16/bf16 -> output [rows, hidden] fp8 (e4m3fnuz as in the reference, or
@@ -193,6 +224,14 @@ TORCH_LIBRARY(_HFRK_C, ops) {
         "skinny_gemm_swiglu(Tensor A, Tensor B, Tensor! act_out, Tensor scale_tensor, Tensor act_scale_tensor, "
         "Tensor! next_buffer, bool mid_bf16) -> ()");
     ops.impl("skinny_gemm_swiglu", torch::kCUDA, &skinny_gemm_swiglu);
+    ops.def(
+        "gate_up_swiglu(Tensor A, Tensor B, Tensor! act_out, Tensor scale_tensor, Tensor act_scale_tensor, "
+        "Tensor! next_buffer, bool mid_bf16) -> ()");
+    ops.impl("gate_up_swiglu", torch::kCUDA, &gate_up_swiglu);
+    ops.def("skinny_gemm_store(Tensor A, Tensor B, Tensor! D, Tensor scale_tensor) -> int");
+    ops.impl("skinny_gemm_store", torch::kCUDA, &skinny_gemm_store);
+    ops.def("skinny_gemm_store_inplace(Tensor A, Tensor B, Tensor! D, Tensor scale_tensor) -> ()");
+    ops.impl("skinny_gemm_store_inplace", torch::kCUDA, &skinny_gemm_store_inplace);
 }
 
 // Shape-only implementations for the Meta key, so that graph tracers (torch.compile, fake tensors)
@@ -205,6 +244,8 @@ int64_t skinny_gemm_tb_meta(torch::Tensor&, torch::Tensor&, torch::Tensor&, torc
 void skinny_gemm_inplace_meta(torch::Tensor&, torch::Tensor&, torch::Tensor&, torch::Tensor&, int64_t) {}
 void skinny_gemm_swiglu_meta(torch::Tensor&, torch::Tensor&, torch::Tensor&, torch::Tensor&, torch::Tensor&,
                              torch::Tensor&, bool) {}
+int64_t skinny_gemm_store_meta(torch::Tensor&, torch::Tensor&, torch::Tensor&, torch::Tensor&) { return HFRK_SUCCESS; }
+void skinny_gemm_store_inplace_meta(torch::Tensor&, torch::Tensor&, torch::Tensor&, torch::Tensor&) {}
 void swiglu_meta(torch::Tensor&, torch::Tensor&, torch::Tensor&, torch::Tensor&, int64_t, bool) {}
 void residual_rms_meta(torch::Tensor&, torch::Tensor&, torch::Tensor&, torch::Tensor&, double, torch::Tensor&,
                        torch::Tensor&, int64_t, bool) {}
@@ -214,6 +255,9 @@ TORCH_LIBRARY_IMPL(_HFRK_C, Meta, ops) {
     ops.impl("skinny_gemm_tb", &skinny_gemm_tb_meta);
     ops.impl("skinny_gemm_inplace", &skinny_gemm_inplace_meta);
     ops.impl("skinny_gemm_swiglu", &skinny_gemm_swiglu_meta);
+    ops.impl("gate_up_swiglu", &skinny_gemm_swiglu_meta);
+    ops.impl("skinny_gemm_store", &skinny_gemm_store_meta);
+    ops.impl("skinny_gemm_store_inplace", &skinny_gemm_store_inplace_meta);
     ops.impl("swiglu", &swiglu_meta);
     ops.impl("residual_rms", &residual_rms_meta);
     ops.impl("increment", &increment_meta);

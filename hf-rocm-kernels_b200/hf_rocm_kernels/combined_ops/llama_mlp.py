@@ -3,9 +3,9 @@
     residual_rms  ->  skinny_gemm (gate/up)  ->  swiglu  ->  skinny_gemm (down)
 
 Same function and argument names as the reference's ``hf_rocm_kernels/combined_ops/llama_mlp.py:7-62``.
-Each element-wise kernel quantises the next GEMM's input and zeroes the buffer that GEMM
-accumulates into, so the chain is four launches with nothing between them; all four are
-programmatic dependents of one another, which lets each GEMM stream weights while the kernel
+Each element-wise kernel quantises the next GEMM's input and the GEMMs store into fresh buffers, so
+the chain is four launches (three with swiglu in the epilogue of the gate/up projection) with nothing
+between them; all are programmatic dependents of one another, which lets each GEMM stream weights while the kernel
 before it is still running.
 
 Two additions for B200: the activations are quantised to the weights' fp8 format (e4m3fnuz as in
@@ -19,8 +19,9 @@ import torch
 from torch import Tensor
 
 import hf_rocm_kernels._HFRK_C  # noqa: F401  (registers torch.ops._HFRK_C)
-from hf_rocm_kernels import residual_rms, skinny_gemm, swiglu
+from hf_rocm_kernels import residual_rms, swiglu
 from hf_rocm_kernels.combined_ops.row_parallel import RowParallelSkinnyGemm
+from hf_rocm_kernels.operators.skinny_gemm.wrapped import skinny_gemm_checks, skinny_gemm_into_empty
 
 
 def can_fuse_swiglu(tokens: int, hidden: int, intermediate: int) -> bool:
@@ -56,6 +57,18 @@ def skinny_gemm_swiglu(
     return out
 
 
+def _gate_up_swiglu(skinny_a: Tensor, gate_up_weight: Tensor, scale_tensor: Tensor, act_scale_tensor: Tensor,
+                    next_buffer: Optional[Tensor], mid_dtype: torch.dtype, out_dtype: torch.dtype) -> Tensor:
+    """:func:`skinny_gemm_swiglu` for any number of tokens."""
+    tokens, inter = skinny_a.size(0), gate_up_weight.size(1) // 2
+    out = torch.empty((tokens, inter), dtype=out_dtype, device=skinny_a.device)
+    if next_buffer is None:
+        next_buffer = torch.empty((tokens, 0), dtype=mid_dtype, device=skinny_a.device)
+    torch.ops._HFRK_C.gate_up_swiglu(skinny_a, gate_up_weight, out, scale_tensor, act_scale_tensor, next_buffer,
+                                     mid_dtype == torch.bfloat16)
+    return out
+
+
 def llama_mlp_combined_ops(
     attn_output: Tensor,
     residual: Tensor,
@@ -88,8 +101,9 @@ def llama_mlp_combined_ops(
         gate_up_gemm_hp, down_gemm_hp: (split_k, b_lanes) pairs of the reference's kernel;
             accepted so that existing callers keep working, not used (the library picks the
             launch shape per (m, n, k), or takes it from its tuning table)
-        fuse_swiglu: run the gate/up projection and swiglu as one launch (same bytes as the two
-            launches); ``None`` decides with :func:`can_fuse_swiglu`
+        fuse_swiglu: run the gate/up projection and swiglu as one launch; ``True`` takes the form of
+            :func:`skinny_gemm_swiglu` (at most 16 tokens, the bytes of the two launches), ``None`` one
+            launch for any number of tokens where rows split into 16-byte pieces
         down_row_parallel: the exchange object of the ranks that share the block; every rank
             multiplies its slice of the swiglu output by its K shard of the down weight and all
             ranks receive the summed result (same bits on every rank)
@@ -99,35 +113,30 @@ def llama_mlp_combined_ops(
     act_dtype = gate_up_weight.dtype
 
     hidden, inter = gate_up_weight.size(0), gate_up_weight.size(1) // 2
-    if fuse_swiglu is None:
-        fuse_swiglu = can_fuse_swiglu(tokens, hidden, inter)
+    # the GEMMs store into fresh buffers; only the row-parallel one adds to what its buffer holds
     mlp_output = torch.empty((tokens, down_weight.size(1)), dtype=attn_output.dtype, device=attn_output.device)
-    if fuse_swiglu:
-        normalized, residual = residual_rms(
-            input=attn_output, residual=residual, weight=rms_weight, epsilon=rms_epsilon,
-            scale_tensor=gate_up_input_scale, next_buffer=None, out_dtype=act_dtype,
-        )
+    zeroed = None if down_row_parallel is None else mlp_output
+    normalized, residual = residual_rms(
+        input=attn_output, residual=residual, weight=rms_weight, epsilon=rms_epsilon,
+        scale_tensor=gate_up_input_scale, next_buffer=None, out_dtype=act_dtype,
+    )
+    if fuse_swiglu is None and (can_fuse_swiglu(tokens, hidden, inter) or (tokens > 16 and inter % 16 == 0)):
+        swiglu_out = _gate_up_swiglu(normalized, gate_up_weight, gate_up_output_scale, down_input_scale, zeroed,
+                                     attn_output.dtype, down_weight.dtype)
+    elif fuse_swiglu:
         swiglu_out = skinny_gemm_swiglu(normalized, gate_up_weight, gate_up_output_scale, down_input_scale,
-                                        next_buffer=mlp_output, mid_dtype=attn_output.dtype,
-                                        out_dtype=down_weight.dtype)
+                                        next_buffer=zeroed, mid_dtype=attn_output.dtype, out_dtype=down_weight.dtype)
     else:
         gate_up_proj = torch.empty((tokens, 2 * inter), dtype=attn_output.dtype, device=attn_output.device)
-        normalized, residual = residual_rms(
-            input=attn_output,
-            residual=residual,
-            weight=rms_weight,
-            epsilon=rms_epsilon,
-            scale_tensor=gate_up_input_scale,
-            next_buffer=gate_up_proj,
-            out_dtype=act_dtype,
-        )
-        skinny_gemm(skinny_a=normalized, b=gate_up_weight, scale_tensor=gate_up_output_scale, output=gate_up_proj)
+        skinny_gemm_checks(normalized, gate_up_weight, gate_up_output_scale, gate_up_proj)
+        skinny_gemm_into_empty(normalized, gate_up_weight, gate_up_output_scale, gate_up_proj)
         swiglu_out = swiglu(
-            gate_up_proj=gate_up_proj, scale_tensor=down_input_scale, next_buffer=mlp_output,
+            gate_up_proj=gate_up_proj, scale_tensor=down_input_scale, next_buffer=zeroed,
             out_dtype=down_weight.dtype,
         )
     if down_row_parallel is None:
-        skinny_gemm(skinny_a=swiglu_out, b=down_weight, scale_tensor=down_output_scale, output=mlp_output)
+        skinny_gemm_checks(swiglu_out, down_weight, down_output_scale, mlp_output)
+        skinny_gemm_into_empty(swiglu_out, down_weight, down_output_scale, mlp_output)
     else:
         assert down_weight.size(0) == swiglu_out.size(1), \
             f"Expected a K shard of {swiglu_out.size(1)} rows but got {down_weight.shape = }"

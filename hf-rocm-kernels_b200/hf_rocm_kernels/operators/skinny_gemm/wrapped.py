@@ -75,6 +75,21 @@ def infer_skinny_gemm_params(skinny_a: Tensor, b: Tensor) -> Dict[str, int]:
     }
 
 
+def _raise_on(status: int) -> None:
+    if status != 0:
+        raise RuntimeError(f"skinny_gemm failed with status {status}: {_STATUS_TEXT.get(status, 'see hfrk_b200.h')}")
+
+
+def skinny_gemm_into_empty(skinny_a: Tensor, b: Tensor, scale_tensor: Tensor, output: Tensor) -> Tensor:
+    """``output = scale_tensor * (skinny_a @ b)`` for a buffer that holds nothing yet: no launch that
+    zeroes it, and the kernel does not read it. The arguments have passed :func:`skinny_gemm_checks`."""
+    if torch.compiler.is_compiling():
+        torch.ops._HFRK_C.skinny_gemm_store_inplace(skinny_a, b, output, scale_tensor)
+    else:
+        _raise_on(torch.ops._HFRK_C.skinny_gemm_store(skinny_a, b, output, scale_tensor))
+    return output
+
+
 def skinny_gemm(
     skinny_a: Tensor,
     b: Tensor,
@@ -88,18 +103,20 @@ def skinny_gemm(
         b: fp8 (k, n) column-major weights, i.e. ``weight_nk.t()`` of a row-major (n, k) matrix.
         scale_tensor: one float32 on the same device, the product of both quantisation scales.
         output: optional (m, n) float16/bfloat16 buffer that already holds zeros or the bias; the
-            result is accumulated into it. Allocated as float16 zeros when omitted.
+            result is accumulated into it. Allocated as float16 when omitted
+            (as if it held zeros).
     Returns:
         ``output``.
     """
     if output is None:
-        output = torch.zeros((skinny_a.size(0), b.size(1)), dtype=torch.float16, device=skinny_a.device)
+        output = torch.empty((skinny_a.size(0), b.size(1)), dtype=torch.float16, device=skinny_a.device)
+        skinny_gemm_checks(skinny_a, b, scale_tensor, output)
+        return skinny_gemm_into_empty(skinny_a, b, scale_tensor, output)
     skinny_gemm_checks(skinny_a, b, scale_tensor, output)
     if torch.compiler.is_compiling():
         # a traced graph cannot hold an op that returns an int: same kernel, raises on a bad status
         torch.ops._HFRK_C.skinny_gemm_inplace(skinny_a, b, output, scale_tensor, 0)
         return output
     status = _skinny_gemm(A=skinny_a, B=b, scale_tensor=scale_tensor, D=output, **infer_skinny_gemm_params(skinny_a, b))
-    if status != 0:
-        raise RuntimeError(f"skinny_gemm failed with status {status}: {_STATUS_TEXT.get(status, 'see hfrk_b200.h')}")
+    _raise_on(status)
     return output

@@ -1,0 +1,173 @@
+"""The GEMM for 17 to 256 tokens per launch with the tokens on the tensor core's M side: plain calls above 64
+tokens (and above 16 in more than one wave), the fused gate/up + swiglu call above 16, store mode."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def capi(native_build):
+    from hf_rocm_kernels import _capi
+
+    return _capi
+
+
+@pytest.fixture(scope="module")
+def dev():
+    return torch.device("cuda:0")
+
+
+def _ok(capi):
+    torch.cuda.synchronize()
+    code, word = capi.device_status(clear=True)
+    assert code == 0, f"device status word {word:#x}"
+
+
+def _operands(m, n, k, fp8, dev):
+    gen = torch.Generator(device=dev).manual_seed(m * 1009 + n * 31 + k)
+    a = torch.randn((m, k), generator=gen, device=dev).to(torch.float8_e4m3fn).view(torch.uint8)
+    w = (torch.randn((n, k), generator=gen, device=dev) * 30).to(torch.float8_e4m3fn).view(torch.uint8)
+    if fp8 == torch.float8_e4m3fnuz:
+        a, w = (torch.where(t == 0x80, torch.zeros_like(t), t) for t in (a, w))
+    return a.view(fp8), w.view(fp8), torch.tensor([1.0 / (30.0 * k ** 0.5)], device=dev)
+
+
+def _bound(ref, a, w, scale, dtype):
+    """One step of the output type, and four standard deviations of the fp32 roundings of a random-walk sum."""
+    step = {torch.float16: 2.0 ** -10, torch.bfloat16: 2.0 ** -7, torch.float32: 2.0 ** -22}[dtype]
+    walk = (a.double().square() @ w.double().square().t()).sqrt() * scale.double().abs()
+    return ref.abs() * step + 4 * 2.0 ** -23 * (a.size(1) / 32 + 1) ** 0.5 * walk + (2.0 ** -24 if dtype == torch.float16 else 0)
+
+
+# one accumulator and two, the edges between them; tiles that end inside the matrix and past it; rows of D
+# that are not 16-byte aligned; a K tail; one K block; K splits of two to six; two launches
+@pytest.mark.parametrize("m,n,k", [(65, 4096, 4096), (128, 6144, 4096), (129, 6144, 4096), (136, 1001, 1040), (256, 28672, 512),
+                                   (255, 4104, 5120), (256, 4096, 14336), (70, 17, 128), (200, 1280, 8192), (130, 33, 16),
+                                   (257, 2000, 2064), (513, 1040, 256), (100, 8192, 1024), (30, 39840, 1024)])
+@pytest.mark.parametrize("fp8,dtype", [(torch.float8_e4m3fn, torch.bfloat16), (torch.float8_e4m3fnuz, torch.float16)])
+def test_wide_gemm_against_float64(capi, dev, m, n, k, fp8, dtype):
+    a, w, scale = _operands(m, n, k, fp8, dev)
+    gen = torch.Generator(device=dev).manual_seed(5)
+    d_in = torch.randn((m, n), generator=gen, device=dev).to(dtype)
+    backing = torch.full((m * n + 64,), 9.0, dtype=dtype, device=dev)
+    d = backing[32:32 + m * n].view(m, n)
+    prod = (a.double() @ w.double().t()) * scale.double()
+    for start, ref in ((d_in, prod + d_in.double()), (torch.zeros_like(d_in), prod)):
+        d.copy_(start)
+        capi.check(capi.skinny_gemm(a, w, d, scale))
+        _ok(capi)
+        assert bool(((d.double() - ref).abs() <= _bound(ref, a, w, scale, dtype)).all())
+    first = d.clone()
+    for _ in range(2):                       # store mode: what D held before does not matter; same bits every time
+        d.fill_(float("nan"))
+        torch.ops._HFRK_C.skinny_gemm_store(a, w.t(), d, scale)
+        _ok(capi)
+        assert torch.equal(d, first)
+    assert bool((backing[:32] == 9).all() and (backing[-32:] == 9).all())
+
+
+def test_wide_gemm_float32_output_and_padded_weights(capi, dev):
+    m, n, k = 150, 1000, 2048
+    a, w, scale = _operands(m, n, k, torch.float8_e4m3fn, dev)
+    padded = torch.zeros((n, k + 48), dtype=torch.uint8, device=dev)
+    padded[:, :k] = w.view(torch.uint8)
+    wp = padded.view(torch.float8_e4m3fn)[:, :k]
+    d = torch.ones((m, n), dtype=torch.float32, device=dev)
+    capi.check(capi.skinny_gemm(a, wp, d, scale))
+    _ok(capi)
+    ref = (a.double() @ w.double().t()) * scale.double() + 1.0
+    assert bool(((d.double() - ref).abs() <= _bound(ref, a, w, scale, torch.float32)).all())
+
+
+@pytest.mark.parametrize("m,inter,k", [(17, 1040, 256), (64, 3584, 8192), (128, 14336, 4096), (129, 2048, 4096), (200, 3584, 8192),
+                                       (256, 28672, 512), (300, 1040, 512), (33, 16, 128), (96, 48, 16)])
+@pytest.mark.parametrize("act,fp8", [(torch.bfloat16, torch.float8_e4m3fn), (torch.float16, torch.float8_e4m3fnuz)])
+def test_wide_gate_up_swiglu_against_the_two_launches(capi, dev, m, inter, k, act, fp8):
+    """The same fp8 values as GEMM + swiglu except where another order of the fp32 sum moves the 16-bit
+    projection across a rounding boundary and that moves the result across one of fp8. A sum over K / 32
+    steps in another order changes by less than 2^-21 of a typical projection, which crosses a 16-bit
+    boundary (2^-8 apart at the coarsest) for at most one value in 2^13 and then moves the product by one
+    16-bit step, across an fp8 boundary (2^-4 apart) in one of 2^4 (bf16) such cases: 2^-17 each for gate and
+    up. Twice that and a margin of eight values for small cases."""
+    from hf_rocm_kernels import skinny_gemm, swiglu
+
+    a, w, scale = _operands(m, 2 * inter, k, fp8, dev)
+    act_scale = torch.tensor([0.02], device=dev)
+    gate_up = torch.zeros((m, 2 * inter), dtype=act, device=dev)
+    skinny_gemm(a, w.t(), scale, gate_up)
+    expect = swiglu(gate_up, act_scale, out_dtype=fp8)
+    backing = torch.full((m * inter + 64,), 0x55, dtype=torch.uint8, device=dev)
+    out = backing[32:32 + m * inter].view(m, inter).view(fp8)
+    zeroed = torch.ones((m, 24), dtype=act, device=dev)
+    torch.ops._HFRK_C.gate_up_swiglu(a, w.t(), out, scale, act_scale, zeroed, act == torch.bfloat16)
+    _ok(capi)
+    differ = int((out.view(torch.uint8) != expect.view(torch.uint8)).sum())
+    assert differ <= 8 + out.numel() * 2.0 ** -15, differ
+    step = (out.float() - expect.float()).abs()
+    assert bool((step <= expect.float().abs() * 2.0 ** -3 + 2.0 ** -9).all())    # one fp8 step
+    assert int(zeroed.count_nonzero()) == 0
+    assert bool((backing[:32] == 0x55).all() and (backing[-32:] == 0x55).all())
+
+
+def test_explicit_launch_shapes_stay_on_the_skinny_kernel(capi, dev):
+    """A requested split or a tuned token bucket means the 64-token launches it was made for."""
+    a, w, scale = _operands(130, 2000, 4096, torch.float8_e4m3fn, dev)
+    ref = (a.double() @ w.double().t()) * scale.double()
+    outs = []
+    for kw in ({"split_k": 3}, {"variant": 1}):
+        d = torch.zeros((130, 2000), dtype=torch.bfloat16, device=dev)
+        capi.check(capi.skinny_gemm_ex(a, w, d, scale, **kw))
+        outs.append(d)
+    capi.lib.hfrk_tuning_set(64, 2000, 4096, 2, 3)
+    try:
+        d = torch.zeros((130, 2000), dtype=torch.bfloat16, device=dev)
+        capi.check(capi.skinny_gemm(a, w, d, scale))
+        outs.append(d)
+    finally:
+        capi.lib.hfrk_tuning_clear()
+    _ok(capi)
+    for d in outs:
+        assert bool(((d.double() - ref).abs() <= _bound(ref, a, w, scale, torch.bfloat16)).all())
+
+
+@pytest.mark.parametrize("tokens", [17, 100, 256])
+@pytest.mark.parametrize("inter", [1040, 1032])            # rows that split into 16-byte pieces, and rows that do not
+def test_mlp_chain_above_16_tokens(capi, dev, tokens, inter):
+    """The chain against itself with swiglu as a launch of its own, eager and from a graph."""
+    from hf_rocm_kernels.combined_ops import llama_mlp_combined_ops
+
+    hidden = 1024
+    gen = torch.Generator(device=dev).manual_seed(3)
+    attn, residual = (torch.randn((tokens, hidden), generator=gen, device=dev).to(torch.bfloat16) for _ in range(2))
+    _, w_gu, s_gu = _operands(1, 2 * inter, hidden, torch.float8_e4m3fn, dev)
+    w_dn = (torch.randn((hidden, (inter + 15) // 16 * 16), generator=gen, device=dev) * 30).to(torch.float8_e4m3fn)[:, :inter]
+    s_dn = torch.tensor([0.02 / (30.0 * inter ** 0.5)], device=dev)
+    one, act_scale = torch.tensor([0.02], device=dev), torch.tensor([0.02], device=dev)
+    norm = torch.ones(hidden, dtype=torch.bfloat16, device=dev)
+
+    def chain(res, **kw):
+        return llama_mlp_combined_ops(attn, res, norm, 1e-5, w_gu.t(), one, s_gu * 0.02, w_dn.t(), act_scale, s_dn, **kw)
+
+    if inter % 16:
+        with pytest.raises(RuntimeError):                  # the down projection's K
+            chain(residual.clone())
+        return
+    out, res = chain(residual.clone())
+    parts, res_parts = chain(residual.clone(), fuse_swiglu=False)
+    with pytest.raises(RuntimeError):
+        chain(residual.clone(), fuse_swiglu=True)
+    _ok(capi)
+    assert torch.equal(res, res_parts)
+    error = (out.double() - parts.double()).norm() / parts.double().norm()
+    assert float(error) <= 2.0 ** -9                       # a few outputs one bf16 step (2^-8) apart at most
+    static, side = residual.clone(), torch.cuda.Stream(dev)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            g_out, _ = chain(static)
+    static.copy_(residual)
+    graph.replay()
+    _ok(capi)
+    assert torch.equal(g_out, out)
