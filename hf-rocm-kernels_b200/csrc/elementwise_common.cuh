@@ -11,6 +11,7 @@
 #include <string.h>
 
 #include "host_common.h"
+#include "ptx_sm100.cuh"
 
 namespace hfrk {
 
@@ -38,6 +39,25 @@ __device__ __forceinline__ uint32_t pack_e4m3x2(float lo, float hi) {
 // utils/fp8.py:26-30 of the reference does.
 __device__ __forceinline__ uint32_t clear_negative_zero_bytes(uint32_t word) {
     return word & ~__vcmpeq4(word, 0x80808080u);
+}
+
+// x / (1 + e^-x) with the accurate expf and an IEEE division: the same expression torch evaluates
+// for silu on fp32 (reference: operators/swiglu/reference.py:18-21).
+__device__ __forceinline__ float silu_f32(float x) { return x / (1.0f + expf(-x)); }
+
+// The same for two values with |x| <= kSiluFastLimit, given as -x, in about half the instructions: the
+// quotient by an approximate reciprocal is corrected once with its exact remainder (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990), two values per
+// instruction. The limit keeps 1 + e^-x far from overflow, where the remainder would be NaN. The
+// reciprocal is taken negative so that a zero keeps its sign. Equal to silu_f32 after the conversion to
+// fp8 for every fp16 and bf16 value (tests/test_gpu_swiglu_fast.py).
+constexpr float kSiluFastLimit = 80.0f;
+__device__ __forceinline__ float2 silu_f32x2(float2 minus_x) {
+    const float2 one = make_float2(1.0f, 1.0f);
+    const float2 d = fma_f32x2(make_float2(expf(minus_x.x), expf(minus_x.y)), one, one);   // 1 + e^-x
+    const float2 minus_r = make_float2(rcp_approx_ftz(-d.x), rcp_approx_ftz(-d.y));
+    const float2 q = mul_f32x2(minus_x, minus_r);
+    return fma_f32x2(fma_f32x2(d, q, minus_x), minus_r, q);
 }
 
 // Zeroes `bytes` bytes (a multiple of 2) starting at `base` (2-byte aligned) with the whole grid.

@@ -246,6 +246,39 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// ---------------------------------------------------------------- packed fp32 arithmetic
+// Two IEEE fp32 operations (round to nearest even, subnormals kept) per instruction.
+__device__ __forceinline__ unsigned long long f32x2_bits(float2 v) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(v.x), "f"(v.y));
+    return r;
+}
+
+__device__ __forceinline__ float2 f32x2_from(unsigned long long r) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
+    return v;
+}
+
+__device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f32x2_bits(a)), "l"(f32x2_bits(b)));
+    return f32x2_from(r);
+}
+
+__device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(f32x2_bits(a)), "l"(f32x2_bits(b)), "l"(f32x2_bits(c)));
+    return f32x2_from(r);
+}
+
+// Reciprocal within one unit in the last place; subnormal arguments and results become zero.
+__device__ __forceinline__ float rcp_approx_ftz(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // ---------------------------------------------------------------- programmatic dependent launch
 // Both are no-ops when the grid was launched without the programmatic-serialisation attribute.
 __device__ __forceinline__ void pdl_wait_prior_grids() {

@@ -84,19 +84,37 @@ static_assert(sizeof(WideCtrl) <= kCtrlBytes, "control block grew");
 // the 16-bit type that the unfused chain stores them in.
 __device__ __forceinline__ uint4 wide_swiglu_16(const float (&gate)[16], const float (&up)[16], float scale, float inv_act,
                                                 int mid_dtype, int fnuz) {
+    float2 g[8], u[8];
+    float top = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        g[i] = make_float2(round_trip_16(gate[2 * i] * scale, mid_dtype), round_trip_16(gate[2 * i + 1] * scale, mid_dtype));
+        u[i] = make_float2(round_trip_16(up[2 * i] * scale, mid_dtype), round_trip_16(up[2 * i + 1] * scale, mid_dtype));
+        top = fmaxf(top, fmaxf(fabsf(g[i].x), fabsf(g[i].y)));   // a NaN does not count, and is one on either path
+    }
     uint32_t words[4];
+    // the fast path encodes e4m3fnuz through twice the scale, which must not overflow
+    if (top <= kSiluFastLimit && inv_act < 1e38f) {
+        const float inv_fast = fnuz ? 2.0f * inv_act : inv_act;
+        const float2 inv = make_float2(inv_fast, inv_fast);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        float t[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float g = round_trip_16(gate[4 * i + j] * scale, mid_dtype);
-            const float u = round_trip_16(up[4 * i + j] * scale, mid_dtype);
-            t[j] = (g / (1.0f + expf(-g))) * u * inv_act;
-            if (fnuz) t[j] *= 2.0f;
+        for (int i = 0; i < 8; ++i) {
+            const float2 t = mul_f32x2(mul_f32x2(silu_f32x2(make_float2(-g[i].x, -g[i].y)), u[i]), inv);
+            const uint32_t pair = pack_e4m3x2(t.x, t.y);
+            words[i >> 1] = (i & 1) == 0 ? pair : words[i >> 1] | (pair << 16);
         }
-        words[i] = pack_e4m3x2(t[0], t[1]) | (pack_e4m3x2(t[2], t[3]) << 16);
-        if (fnuz) words[i] = clear_negative_zero_bytes(words[i]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float2 t = make_float2(silu_f32(g[i].x) * u[i].x * inv_act, silu_f32(g[i].y) * u[i].y * inv_act);
+            if (fnuz) t = make_float2(t.x * 2.0f, t.y * 2.0f);
+            const uint32_t pair = pack_e4m3x2(t.x, t.y);
+            words[i >> 1] = (i & 1) == 0 ? pair : words[i >> 1] | (pair << 16);
+        }
+    }
+    if (fnuz) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) words[i] = clear_negative_zero_bytes(words[i]);
     }
     return make_uint4(words[0], words[1], words[2], words[3]);
 }
