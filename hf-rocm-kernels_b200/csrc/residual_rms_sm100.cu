@@ -223,11 +223,16 @@ residual_rms_scalar_kernel(const T* __restrict__ input, T* __restrict__ residual
 
 // CTA size. A hint that is a multiple of 32 is taken as it is. Otherwise one work item (a 16-byte
 // vector, or an element on the scalar path) per thread: the shortest critical path, which is what
-// the few rows of a decode step need. With more rows than the machine holds CTAs at once, two items
-// per thread: smaller CTAs, more of them per SM, so one CTA's reduction overlaps another's loads.
+// the few rows of a decode step need. Two items per thread, i.e. smaller CTAs,
+//   * with more rows than the machine holds CTAs at once: more CTAs per SM, so one CTA's reduction
+//     overlaps another's loads;
+//   * with more rows than SMs where one item per thread means more than 512 threads: two such CTAs do
+//     not fit on an SM (64 registers per thread), which makes two waves (200 x 8192: 5.3 -> 3.8 us).
+// For a few rows of 513 to 1024 vectors two items are faster alone (4 x 8192: 2.6 -> 2.3 us) but slower
+// between the GEMMs of a decode step (four layers of a 70B shard at 16 tokens: 154.0 -> 157.1 us).
 int choose_threads(int work_items, int rows, int hint) {
     if (hint >= 32 && hint <= 1024 && hint % 32 == 0) return hint;
-    if (rows > 2 * kSmCount) work_items = (work_items + 1) / 2;
+    if (rows > 2 * kSmCount || (rows > kSmCount && work_items > 512)) work_items = (work_items + 1) / 2;
     int threads = ((work_items + 31) / 32) * 32;
     if (threads < 64) threads = 64;
     if (threads > 1024) threads = 1024;
