@@ -57,6 +57,17 @@ def skinny_gemm_swiglu(
     return out
 
 
+def _fuses(tokens: int, hidden: int, intermediate: int) -> bool:
+    """Whether the block folds swiglu into the gate/up projection when the caller does not say. Above 16
+    tokens that is the kernel with the tokens on the tensor core's M side, which starts some 2 us later
+    than the projection alone would: it saves a launch of 3 us, but a small matrix at few tokens gains
+    nothing (20 tokens, 9216 x 1568: four layers 113 us in two launches, 119 us in one; 26 tokens,
+    11168 x 2192: 147 and 145 us)."""
+    if intermediate % 16 != 0:
+        return False
+    return tokens <= 16 or tokens > 32 or 2 * intermediate * hidden >= 20_000_000
+
+
 def _gate_up_swiglu(skinny_a: Tensor, gate_up_weight: Tensor, scale_tensor: Tensor, act_scale_tensor: Tensor,
                     next_buffer: Optional[Tensor], mid_dtype: torch.dtype, out_dtype: torch.dtype) -> Tensor:
     """:func:`skinny_gemm_swiglu` for any number of tokens."""
@@ -120,7 +131,7 @@ def llama_mlp_combined_ops(
         input=attn_output, residual=residual, weight=rms_weight, epsilon=rms_epsilon,
         scale_tensor=gate_up_input_scale, next_buffer=None, out_dtype=act_dtype,
     )
-    if fuse_swiglu is None and (can_fuse_swiglu(tokens, hidden, inter) or (tokens > 16 and inter % 16 == 0)):
+    if fuse_swiglu is None and _fuses(tokens, hidden, inter):
         swiglu_out = _gate_up_swiglu(normalized, gate_up_weight, gate_up_output_scale, down_input_scale, zeroed,
                                      attn_output.dtype, down_weight.dtype)
     elif fuse_swiglu:
