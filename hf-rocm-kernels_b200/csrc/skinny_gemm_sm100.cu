@@ -610,7 +610,7 @@ struct WideReq {
 // latency of a load over the stages that hide it. To it come the fixed cost of a call in a chain of
 // dependent calls, one per further wave, the epilogue's stores and, with a K split, the cluster barrier
 // and the partials that a CTA sends to its peers (~40 GB/s per SM). The constants are a fit to
-// 3,900 timings on a B200 (114 shapes of 17 to 256 tokens, every tile height, split and CTAs per SM that
+// 10,400 timings on a B200 (148 shapes of 17 to 256 tokens, every tile height, split and CTAs per SM that
 // fits): the shape it picks is on average 4.5 % slower than the best of its list, 26 % at worst.
 struct WideCost {
     int n, k, halves, rows, tile_n, split, stages, per_sm, ctas, waves, ctas_busiest, kb;
@@ -717,8 +717,11 @@ int make_wide_plan(const DeviceModel& dm, int m, int n, int k, bool swiglu, cons
 // the skinny kernel:
 //   * more tokens than one launch of the skinny kernel holds: 28672 x 4096 at 256 tokens 31 us against 91;
 //   * 17 to 64 tokens where the skinny kernel's unsplit grid needs a second wave, because its activation
-//     tile leaves room for two CTAs per SM: 39840 x 6272 at 30 tokens 42 us against 55. In one wave the
-//     two are within a few percent of each other, and up to 16 tokens the skinny kernel is always ahead.
+//     tile leaves room for two CTAs per SM: 39840 x 6272 at 30 tokens 42 us against 55;
+//   * 33 to 64 tokens where an owner of its K split finishes more than kOwned token rows and the
+//     reduction runs past its registers, D_in late: 6144 x 4096 at 64 tokens 9.9 us against 12.3,
+//     10240 x 8192 19.2 against 29.1, 8192 x 8192 16.2 against 17.7; overwriting D, the two are even.
+// Elsewhere up to 64 tokens the skinny kernel is ahead (by 1 to 3 us, most at the fewest tokens).
 bool use_wide_kernel(const DeviceModel& dm, int m, int n, int k, bool explicit_shape) {
     if (explicit_shape || m <= 16) return false;
     TuneValue tuned;
@@ -727,7 +730,7 @@ bool use_wide_kernel(const DeviceModel& dm, int m, int n, int k, bool explicit_s
     if (m > kMaxMPad) return true;
     Plan plan;
     if (make_plan(dm, m, n, k, 0, 0, &plan) != HFRK_SUCCESS) return false;
-    return plan.split == 1 && plan.ctas > ctas_per_sm(plan.smem_bytes) * dm.sms;
+    return plan.split == 1 ? plan.ctas > ctas_per_sm(plan.smem_bytes) * dm.sms : (1 << plan.rows_log2) > kOwned;
 }
 
 // One launch per 256 tokens, the tokens shared out evenly. The caller has validated the arguments.
