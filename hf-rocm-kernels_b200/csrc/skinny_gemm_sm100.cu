@@ -229,7 +229,7 @@ constexpr BuiltinShape kBuiltinShapes[] = {
 //   * three CTAs per SM (a ring of three 18 KiB stages) beat two (four stages) on most shapes:
 //     the third slot lets part of the NEXT call's grid move in and start its weight stream while
 //     this call drains;
-//   * at least two K blocks per CTA; no split once the tiles alone cover the SMs (then six
+//   * at least two K blocks per CTA once the CTAs outnumber the SMs; no split once the tiles alone cover the SMs (then six
 //     stages, two CTAs per SM, or three stages when that saves a wave: 448 tiles on 444 slots);
 //   * tiles of fewer than 128 rows even out a grid without a K split that is between one and two
 //     CTAs per SM: 224 tiles of 128 rows put two CTAs on 76 SMs and one on the other 72; 256
@@ -254,8 +254,10 @@ int make_plan(const DeviceModel& dm, int m, int n, int k, int split_req, int sta
         const int smem = plan_smem_bytes(m, m_pad, split, stages);
         if (smem > kSmemLimit) return false;
         const int per_sm = ctas_per_sm(smem) < max_per_sm ? ctas_per_sm(smem) : max_per_sm;
-        // one cluster to spare: at the exact capacity a straggler of the previous grid keeps the last one out
-        return per_sm >= 1 && tiles < dm.capacity[split][per_sm];
+        // one cluster to spare, up to 16 tokens (three CTAs per SM, shorter calls) two: closer to the capacity a
+        // straggler of the previous grid keeps the last ones out (10336 x 6992 as 81 clusters of 5 where 82 fit: 17.0 us, 14.5 with clusters of 4; 3792 x 11792 as 30
+        // clusters of 12 where 31 fit: 11.6 us, 10.0 with clusters of 9)
+        return per_sm >= 1 && tiles + (m_pad == 16 ? 2 : 1) <= dm.capacity[split][per_sm];
     };
 
     TuneValue tuned;
@@ -293,8 +295,11 @@ int make_plan(const DeviceModel& dm, int m, int n, int k, int split_req, int sta
             const int ring_choices[3] = {2, 3, 4};
             for (int choice = m_pad > 16 ? 0 : 1; choice < 3; ++choice) {
                 const int ring = stages_req != 0 ? stages_req : ring_choices[choice];
+                // Up to 16 tokens one K block per CTA is enough while the CTAs do not fill the SMs (1104 x 1104:
+                // 3.4 us with clusters of 4, 2.9 with clusters of 9).
                 for (int s = kMaxSplit; s >= 2; --s) {
-                    if (nkb / s < 2) continue;
+                    const bool few = m_pad == 16 && s <= nkb && tiles * s <= dm.sms;
+                    if (nkb / s < 2 && !few) continue;
                     if (!resident(s, ring)) continue;
                     const int ctas = tiles * s;
                     bool better;

@@ -1,5 +1,5 @@
-"""The GEMM for 17 to 256 tokens per launch with the tokens on the tensor core's M side: plain calls above 64
-tokens (and above 16 in more than one wave), the fused gate/up + swiglu call above 16, store mode."""
+"""Automatic launch shapes against float64: the GEMM for 17 to 256 tokens per launch with the tokens on the tensor core's M side: plain calls above 64
+tokens (and above 16 in more than one wave), the fused gate/up + swiglu call above 16, store mode, and some small shapes of the skinny kernel."""
 import pytest
 import torch
 
@@ -44,7 +44,10 @@ def _bound(ref, a, w, scale, dtype):
 # that are not 16-byte aligned; a K tail; one K block; K splits of two to six; two launches
 @pytest.mark.parametrize("m,n,k", [(65, 4096, 4096), (128, 6144, 4096), (129, 6144, 4096), (136, 1001, 1040), (256, 28672, 512),
                                    (255, 4104, 5120), (256, 4096, 14336), (70, 17, 128), (200, 1280, 8192), (130, 33, 16),
-                                   (257, 2000, 2064), (513, 1040, 256), (100, 8192, 1024), (30, 39840, 1024)])
+                                   (257, 2000, 2064), (513, 1040, 256), (100, 8192, 1024), (30, 39840, 1024),
+                                   # up to 16 tokens: K splits down to one K block per CTA (few tiles), and the
+                                   # grids that stay two clusters below the device's capacity
+                                   (4, 1104, 1104), (16, 1808, 1808), (3, 17, 256), (11, 10336, 6992)])
 @pytest.mark.parametrize("fp8,dtype", [(torch.float8_e4m3fn, torch.bfloat16), (torch.float8_e4m3fnuz, torch.float16)])
 def test_wide_gemm_against_float64(capi, dev, m, n, k, fp8, dtype):
     a, w, scale = _operands(m, n, k, fp8, dev)
