@@ -244,7 +244,9 @@ int hfrk_skinny_gemm_fp8_profile(const void* A, const void* W, void* D, const fl
 /* Launch shape for (m, n, k) and the given pins (for logs and tests; no GPU work).
  * out[0]=variant chosen, out[1]=split_k (0 for STREAMK), out[2]=num_stages, out[3]=grid CTAs,
  * out[4]=dynamic shared memory bytes, out[5]=padded token count (MMA N), out[6]=K blocks of 128,
- * out[7]=tiles along N (of out[3]/out[1] CTAs; a tile is at most 128 rows). Returns a status code. */
+ * out[7]=tiles along N (of out[3]/out[1] CTAs; a tile is at most 128 rows). Describes the kernel that pins
+ * apply to, in launches of at most 64 tokens; automatic calls with more tokens (and some from 17 on)
+ * run the wide kernel, whose shape follows from (m, n, k) and the device. Returns a status code. */
 int hfrk_skinny_gemm_plan(int m, int n, int k, int variant, int split_k, int ctas_per_sm, int* out8);
 
 /* ---- the element-wise kernels either side of the GEMM in a decoder layer -------------------
