@@ -249,15 +249,17 @@ int make_plan(const DeviceModel& dm, int m, int n, int k, int split_req, int sta
     const int stage_bytes = kWStageBytes + m_pad * kBlockK;
     const int two_per_sm = 2 * dm.sms;
 
-    // all clusters of (split, stages) resident at once on this device?
-    auto resident = [&](int split, int stages) {
+    // all clusters of (split, stages) resident at once on this device, with room for `spare` more?
+    auto resident = [&](int split, int stages, int spare) {
         const int smem = plan_smem_bytes(m, m_pad, split, stages);
         if (smem > kSmemLimit) return false;
         const int per_sm = ctas_per_sm(smem) < max_per_sm ? ctas_per_sm(smem) : max_per_sm;
-        // one cluster to spare, up to 16 tokens (three CTAs per SM, shorter calls) two: closer to the capacity a
-        // straggler of the previous grid keeps the last ones out (10336 x 6992 as 81 clusters of 5 where 82 fit: 17.0 us, 14.5 with clusters of 4; 3792 x 11792 as 30
-        // clusters of 12 where 31 fit: 11.6 us, 10.0 with clusters of 9)
-        return per_sm >= 1 && tiles + (m_pad == 16 ? 2 : 1) <= dm.capacity[split][per_sm];
+        // At the exact capacity a straggler of the previous grid keeps the last cluster out: one stays free. Shapes
+        // of the rule that put three CTAs on an SM (up to 16 tokens) leave two: with a single one the last cluster
+        // still starts late there (10336 x 6992 as 81 clusters of 5 where 82 fit: 17.0 us, 14.5 with clusters
+        // of 4; 3792 x 11792 as 30 clusters of 12 where 31 fit: 11.6 us, 10.0 with clusters of 9).
+        if (spare > 1 && (m_pad != 16 || per_sm < 3)) spare = 1;
+        return per_sm >= 1 && tiles + spare <= dm.capacity[split][per_sm];
     };
 
     TuneValue tuned;
@@ -268,7 +270,8 @@ int make_plan(const DeviceModel& dm, int m, int n, int k, int split_req, int sta
             tile_rows_req = tuned.tile_rows;
         } else if (m_pad == 16) {
             for (const BuiltinShape& b : kBuiltinShapes) {
-                if (b.n == n && b.k == k && (b.split == 1 || resident(b.split, b.stages))) {
+                // measured with one cluster to spare (4096 x 14336 as 32 clusters of 8 where 33 fit: 11.9 us, 12.5 as 12 x 3)
+                if (b.n == n && b.k == k && (b.split == 1 || resident(b.split, b.stages, 1))) {
                     split_req = b.split;
                     stages_req = b.stages;
                     break;
@@ -300,7 +303,7 @@ int make_plan(const DeviceModel& dm, int m, int n, int k, int split_req, int sta
                 for (int s = kMaxSplit; s >= 2; --s) {
                     const bool few = m_pad == 16 && s <= nkb && tiles * s <= dm.sms;
                     if (nkb / s < 2 && !few) continue;
-                    if (!resident(s, ring)) continue;
+                    if (!resident(s, ring, 2)) continue;
                     const int ctas = tiles * s;
                     bool better;
                     if (m_pad > 16) {

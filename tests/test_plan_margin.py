@@ -10,9 +10,10 @@ def capi(native_build):
 
 
 def _plan(capi, m, n, k, capacity):
+    """``capacity``: per split the clusters that fit with three CTAs on an SM, or (one, two, three) of them."""
     table = [[0, 0, 0, 0]] + [[0] + [148 * per_sm // split for per_sm in (1, 2, 3)] for split in range(1, 17)]
     for split, value in capacity.items():
-        table[split] = [0, value // 3, value * 2 // 3, value]
+        table[split] = [0, *value] if isinstance(value, tuple) else [0, value // 3, value * 2 // 3, value]
     capi.override_device_model(148, table)
     try:
         return capi.plan(m, n, k)
@@ -31,3 +32,18 @@ def test_two_clusters_stay_free(capi, spare, split):
 def test_one_k_block_per_cta_while_sms_are_idle(capi, n, k, split):
     """9 tiles x 9 K blocks and 15 x 9 CTAs fit on 148 SMs; 27 tiles do not, and keep two K blocks per CTA."""
     assert _plan(capi, 16, n, k, {})["split_k"] == split
+
+
+@pytest.mark.parametrize("m", [1, 4, 16])
+@pytest.mark.parametrize("fit,shape", [(33, (8, 5)), (34, (8, 5)), (32, None)])
+def test_a_measured_shape_needs_one_free_cluster(capi, m, fit, shape):
+    """The 8B down projection was measured as 32 clusters of 8 at two CTAs per SM on chips that hold 33."""
+    got = _plan(capi, m, 4096, 14336, {8: (16, fit, 50)})
+    assert ((got["split_k"], got["num_stages"]) == (8, 5)) == (shape is not None)
+
+
+@pytest.mark.parametrize("spare,split", [(0, 4), (1, 5), (2, 5)])
+def test_one_cluster_stays_free_at_two_ctas_per_sm(capi, spare, split):
+    """Two CTAs per SM (nothing larger than 5 fits, nothing at all at three per SM): 40 tiles need room for 41."""
+    none = {s: (0, 0, 0) for s in (2, 3, *range(6, 17))}
+    assert _plan(capi, 16, 5120, 9600, {**none, 4: (37, 74, 0), 5: (20, 40 + spare, 0)})["split_k"] == split
