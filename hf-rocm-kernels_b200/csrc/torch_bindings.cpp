@@ -101,6 +101,11 @@ static void call_gate_up_swiglu(GateUpEntry entry, torch::Tensor& A, torch::Tens
     TORCH_CHECK(next_buffer.is_contiguous() && next_buffer.element_size() == 2 &&
                     (next_buffer.numel() == 0 || next_buffer.size(0) == m),
                 "skinny_gemm_swiglu: next_buffer must be a contiguous 16-bit [m, .] matrix");
+    // the kernel dereferences all six: a host tensor among them would be a bad address
+    for (const torch::Tensor* t : {&A, &B, &act_out, &scale_tensor, &act_scale_tensor, &next_buffer}) {
+        TORCH_CHECK(t->numel() == 0 || (t->is_cuda() && t->device() == A.device()), "skinny_gemm_swiglu: all tensors must be on one GPU, got ",
+                    t->device(), " and ", A.device());
+    }
     TORCH_CHECK(m <= INT32_MAX && inter <= INT32_MAX && k <= INT32_MAX, "skinny_gemm_swiglu: extent above 2^31");
     const at::cuda::OptionalCUDAGuard device_guard(device_of(A));
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream();

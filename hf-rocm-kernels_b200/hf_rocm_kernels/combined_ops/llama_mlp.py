@@ -21,7 +21,8 @@ from torch import Tensor
 import hf_rocm_kernels._HFRK_C  # noqa: F401  (registers torch.ops._HFRK_C)
 from hf_rocm_kernels import residual_rms, swiglu
 from hf_rocm_kernels.combined_ops.row_parallel import RowParallelSkinnyGemm
-from hf_rocm_kernels.operators.skinny_gemm.wrapped import skinny_gemm_checks, skinny_gemm_into_empty
+from hf_rocm_kernels.operators.skinny_gemm.wrapped import (skinny_gemm_checks, skinny_gemm_into_empty,
+                                                           skinny_gemm_operand_checks)
 
 
 def can_fuse_swiglu(tokens: int, hidden: int, intermediate: int) -> bool:
@@ -70,8 +71,16 @@ def _fuses(tokens: int, hidden: int, intermediate: int) -> bool:
 
 def _gate_up_swiglu(skinny_a: Tensor, gate_up_weight: Tensor, scale_tensor: Tensor, act_scale_tensor: Tensor,
                     next_buffer: Optional[Tensor], mid_dtype: torch.dtype, out_dtype: torch.dtype) -> Tensor:
-    """:func:`skinny_gemm_swiglu` for any number of tokens."""
+    """:func:`skinny_gemm_swiglu` for any number of tokens. Above 16 tokens it stands in for two launches
+    through ``skinny_gemm`` and ``swiglu`` and refuses what their checks refuse, as they do."""
     tokens, inter = skinny_a.size(0), gate_up_weight.size(1) // 2
+    if tokens > 16:
+        skinny_gemm_operand_checks(skinny_a, gate_up_weight, scale_tensor)
+        assert gate_up_weight.size(1) % 2 == 0, f"Expected an even number of columns: {gate_up_weight.shape = }."
+        assert act_scale_tensor.numel() == 1, f"Expected {act_scale_tensor.numel() = } to be 1."
+        assert act_scale_tensor.device == skinny_a.device, \
+            f"Expected {act_scale_tensor.device = } to be the same as {skinny_a.device = }"
+        assert out_dtype in (torch.float8_e4m3fn, torch.float8_e4m3fnuz), f"Expected an e4m3 {out_dtype = }"
     out = torch.empty((tokens, inter), dtype=out_dtype, device=skinny_a.device)
     if next_buffer is None:
         next_buffer = torch.empty((tokens, 0), dtype=mid_dtype, device=skinny_a.device)
