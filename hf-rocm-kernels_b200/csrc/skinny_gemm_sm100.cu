@@ -1417,12 +1417,15 @@ namespace {
 constexpr size_t kBatchMergeBytes = 512 * 1024;   // largest merged activation copy; smallest result group
 constexpr int kBatchEvents = 64;
 
-// Per device: the library's copy streams, one per direction, and a ring of events (an event may be
+// Per device: the library's copy streams, one per direction, and two rings of events (an event may be
 // recorded again while an older wait on it is pending: a wait refers to the record that preceded it).
+// Events of `in_events` are recorded on the inbound stream only, so that one that was recorded again before
+// its call waits for it stands for a later point of the same stream, which covers the earlier one. Events of
+// `events` are waited for right after they are recorded.
 struct BatchResources {
     cudaStream_t in_stream = nullptr, out_stream = nullptr;
-    cudaEvent_t events[kBatchEvents] = {};
-    int next_event = 0;
+    cudaEvent_t events[kBatchEvents] = {}, in_events[kBatchEvents] = {};
+    int next_event = 0, next_in_event = 0;
     bool ready = false;
 };
 std::mutex g_batch_mutex;
@@ -1437,7 +1440,9 @@ int batch_resources(BatchResources** out) {
         if (r.in_stream == nullptr) HFRK_CUDA_TRY(cudaStreamCreateWithFlags(&r.in_stream, cudaStreamNonBlocking));
         if (r.out_stream == nullptr) HFRK_CUDA_TRY(cudaStreamCreateWithFlags(&r.out_stream, cudaStreamNonBlocking));
         for (int i = 0; i < kBatchEvents; ++i) {
-            HFRK_CUDA_TRY(cudaEventCreateWithFlags(&r.events[i], cudaEventDisableTiming));
+            for (cudaEvent_t* e : {&r.events[i], &r.in_events[i]}) {
+                if (*e == nullptr) HFRK_CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+            }
         }
         r.ready = true;
     }
@@ -1453,8 +1458,43 @@ bool batch_call_valid(const hfrk_host_call& c) {
            c.n > 0 && c.k > 0 && (c.d_dtype == HFRK_F16 || c.d_dtype == HFRK_BF16 || c.d_dtype == HFRK_F32);
 }
 
+// True if the result of a call lands where a later call's activations or D_in are read from. The bounding
+// box of the results so far spares the usual list (results in blocks of their own) the comparison by pairs.
+bool batch_overwrites_inputs(const hfrk_host_call* calls, int count) {
+    uintptr_t lo = UINTPTR_MAX, hi = 0;
+    auto result_bytes = [&](int i) {
+        return static_cast<size_t>(calls[i].m) * calls[i].n * out_elem_bytes(calls[i].d_dtype);
+    };
+    auto overwritten = [&](const void* input, size_t bytes, int before) {
+        const uintptr_t from = reinterpret_cast<uintptr_t>(input), to = from + bytes;
+        if (to <= lo || from >= hi) return false;
+        for (int i = 0; i < before; ++i) {
+            const uintptr_t d = reinterpret_cast<uintptr_t>(calls[i].D_host);
+            if (from < d + result_bytes(i) && d < to) return true;
+        }
+        return false;
+    };
+    for (int i = 0; i < count; ++i) {
+        const hfrk_host_call& c = calls[i];
+        if (overwritten(c.A_host, static_cast<size_t>(c.m) * c.k, i)) return true;
+        if (c.accumulate && overwritten(c.D_in_host != nullptr ? c.D_in_host : c.D_host, result_bytes(i), i)) return true;
+        const uintptr_t d = reinterpret_cast<uintptr_t>(c.D_host);
+        if (d < lo) lo = d;
+        if (d + result_bytes(i) > hi) hi = d + result_bytes(i);
+    }
+    return false;
+}
+
 }  // namespace
 }  // namespace hfrk
+
+extern "C" int hfrk_host_batch_inputs_first(const hfrk_host_call* calls, int count) {
+    if (calls == nullptr || count <= 0) return 0;
+    for (int i = 0; i < count; ++i) {
+        if (!hfrk::batch_call_valid(calls[i])) return 0;
+    }
+    return hfrk::batch_overwrites_inputs(calls, count) ? 1 : 0;
+}
 
 extern "C" int64_t hfrk_host_batch_workspace_bytes(const hfrk_host_call* calls, int count) {
     if (calls == nullptr || count <= 0) return 0;
@@ -1485,6 +1525,12 @@ extern "C" int hfrk_skinny_gemm_fp8_host_batch(const hfrk_host_call* calls, int 
     auto next_event = [&]() {
         cudaEvent_t e = res->events[res->next_event];
         res->next_event = (res->next_event + 1) % kBatchEvents;
+        return e;
+    };
+
+    auto next_in_event = [&]() {
+        cudaEvent_t e = res->in_events[res->next_in_event];
+        res->next_in_event = (res->next_in_event + 1) % kBatchEvents;
         return e;
     };
 
@@ -1554,7 +1600,7 @@ extern "C" int hfrk_skinny_gemm_fp8_host_batch(const hfrk_host_call* calls, int 
             }
             sent_d_off += align16(bytes);
         }
-        cudaEvent_t e = next_event();
+        cudaEvent_t e = next_in_event();
         HFRK_CUDA_TRY(cudaEventRecord(e, res->in_stream));
         needs_event[i] = e;
         sent_off += run;
@@ -1562,7 +1608,20 @@ extern "C" int hfrk_skinny_gemm_fp8_host_batch(const hfrk_host_call* calls, int 
         return HFRK_SUCCESS;
     };
 
-    // Results leave on the outbound stream in at most eight groups of at least kBatchMergeBytes: each
+    // Every input of the list is read before any result is written. With results in blocks of their own the
+    // order of the two streams does not matter; a list that writes a result over a later call's input (calls that
+    // accumulate into one block, an activation block that another call fills) has all inputs read first.
+    if (batch_overwrites_inputs(calls, count)) {
+        while (sent < count) {
+            rc = send_chunk();
+            if (rc != HFRK_SUCCESS) return rc;
+        }
+        cudaEvent_t e = next_event();
+        HFRK_CUDA_TRY(cudaEventRecord(e, res->in_stream));
+        HFRK_CUDA_TRY(cudaStreamWaitEvent(res->out_stream, e, 0));
+    }
+
+    // Results leave on the outbound stream in groups of at least an eighth of them and kBatchMergeBytes: each
     // group's copy overlaps the GEMMs after it and the inbound copies, and every group costs one
     // dependency between the streams. Three groups left the copies idle until a third of the step was
     // done and 48 us of them to do after the last GEMM.

@@ -35,7 +35,7 @@ EXPORTED_SYMBOLS = (
     "hfrk_skinny_gemm_fp8_noalloc", "hfrk_max_active_clusters", "hfrk_tuning_set", "hfrk_tuning_clear",
     "hfrk_swiglu_fp8", "hfrk_residual_rms", "hfrk_rowpar_set_mode",
     "hfrk_skinny_gemm_fp8_swiglu", "hfrk_gate_up_swiglu_fp8", "hfrk_skinny_gemm_fp8_host_async",
-    "hfrk_tuning_set_ex", "hfrk_rowpar_set_wait_ms", "hfrk_device_model_get", "hfrk_device_model_override",
+    "hfrk_tuning_set_ex", "hfrk_host_batch_inputs_first", "hfrk_rowpar_set_wait_ms", "hfrk_device_model_get", "hfrk_device_model_override",
 )
 
 
@@ -121,6 +121,8 @@ class HostCall(ctypes.Structure):
 lib = _load()
 lib.hfrk_host_batch_workspace_bytes.argtypes = [ctypes.POINTER(HostCall), ctypes.c_int]
 lib.hfrk_host_batch_workspace_bytes.restype = ctypes.c_int64
+lib.hfrk_host_batch_inputs_first.argtypes = [ctypes.POINTER(HostCall), ctypes.c_int]
+lib.hfrk_host_batch_inputs_first.restype = ctypes.c_int
 lib.hfrk_skinny_gemm_fp8_host_batch.argtypes = [ctypes.POINTER(HostCall), ctypes.c_int, ctypes.c_void_p, ctypes.c_int64,
                                                 ctypes.c_void_p]
 lib.hfrk_skinny_gemm_fp8_host_batch.restype = ctypes.c_int

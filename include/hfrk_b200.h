@@ -126,14 +126,17 @@ int hfrk_skinny_gemm_fp8_host_async(const void* A_host, const void* W_dev, void*
 /* One decode step's worth of host-buffer calls in ONE library call. A caller that drives the GEMMs
  * one by one from an interpreter pays more for submitting a call than the GPU needs to run it; here
  * the whole list is queued by one native loop:
- *   * activations go host->device on a copy stream owned by the library, neighbouring host blocks
- *     merged into copies of up to 512 KiB (one cudaMemcpyAsync per merged block, D_in of the
- *     block's accumulating calls behind it), each followed by an event that `stream` waits for
- *     only before the first GEMM that needs it;
+ *   * activations go host->device on an inbound copy stream owned by the library, neighbouring host
+ *     blocks merged into copies of up to about 512 KiB (one cudaMemcpyAsync per merged block, D_in of
+ *     the block's accumulating calls behind it), submitted one block ahead of the calls that use
+ *     them, each followed by an event that `stream` waits for only before the first GEMM that needs it;
  *   * nothing but the GEMMs runs on `stream`, in list order, so consecutive calls overlap as they
  *     do for device-resident callers;
- *   * results go device->host on the copy stream in about three groups, each behind an event
- *     recorded after the group's last GEMM, so that a group's copy overlaps the next group's GEMMs;
+ *   * results go device->host on an outbound copy stream in groups of at least an eighth of them (and
+ *     512 KiB), the last two or three calls each as a group of its own, each behind an event recorded
+ *     after the group's last GEMM, so that a group's copy overlaps the GEMMs after it;
+ *   * every A_host and D_in of the list is read before any D_host is written. Lists whose D_host blocks
+ *     overlap inputs of later calls (hfrk_host_batch_inputs_first) are submitted with all inputs first;
  *   * `stream` finally waits for the last copy: the caller synchronises `stream` once and finds
  *     every D_host filled.
  * work_dev: device scratch of at least hfrk_host_batch_workspace_bytes(calls, count) bytes; host
@@ -154,6 +157,9 @@ typedef struct hfrk_host_call {
                               * D_host before every step. */
 } hfrk_host_call;
 int64_t hfrk_host_batch_workspace_bytes(const hfrk_host_call* calls, int count);
+/* 1 if some call's D_host overlaps the A_host or the D_in block of a later call, so that the batch reads
+ * all inputs before its first result leaves; 0 otherwise (no GPU work). */
+int hfrk_host_batch_inputs_first(const hfrk_host_call* calls, int count);
 int hfrk_skinny_gemm_fp8_host_batch(const hfrk_host_call* calls, int count, void* work_dev,
                                     int64_t work_bytes, void* stream);
 
