@@ -1453,6 +1453,26 @@ int batch_resources(BatchResources** out) {
 size_t out_elem_bytes(int d_dtype) { return d_dtype == HFRK_F32 ? 4 : 2; }
 size_t align16(size_t v) { return (v + 15) & ~static_cast<size_t>(15); }
 
+// Makes the caller's stream wait for both copy streams when a batch ends early: what was submitted before the
+// failing call still reads and writes the caller's host blocks and scratch, and the next batch on that scratch
+// waits for the caller's stream alone.
+struct BatchJoin {
+    BatchResources* res;
+    cudaStream_t stream;
+    bool in_used = false, out_used = false, complete = false;
+    ~BatchJoin() {
+        if (complete) return;
+        if (in_used) join(res->in_stream);
+        if (out_used) join(res->out_stream);
+    }
+    void join(cudaStream_t copies) {
+        cudaEvent_t e = res->events[res->next_event];
+        res->next_event = (res->next_event + 1) % kBatchEvents;
+        if (cudaEventRecord(e, copies) != cudaSuccess || cudaStreamWaitEvent(stream, e, 0) != cudaSuccess)
+            (void)cudaGetLastError();   // the call that ended the batch is the one to report
+    }
+};
+
 bool batch_call_valid(const hfrk_host_call& c) {
     return c.A_host != nullptr && c.W_dev != nullptr && c.D_host != nullptr && c.scale_dev != nullptr && c.m > 0 &&
            c.n > 0 && c.k > 0 && (c.d_dtype == HFRK_F16 || c.d_dtype == HFRK_BF16 || c.d_dtype == HFRK_F32);
@@ -1546,11 +1566,13 @@ extern "C" int hfrk_skinny_gemm_fp8_host_batch(const hfrk_host_call* calls, int 
     // first kept the GPU waiting for its first GEMM for 33 us of host time (16 calls of a Llama-3 8B step).
     cudaEvent_t needs_event[1024] = {};
     if (count > 1024) return HFRK_TOO_LARGE;
+    BatchJoin join{res, s};
     {
         // the scratch may still be in use by what was queued on `stream` before (the previous batch)
         cudaEvent_t before = next_event();
         HFRK_CUDA_TRY(cudaEventRecord(before, s));
         HFRK_CUDA_TRY(cudaStreamWaitEvent(res->in_stream, before, 0));
+        join.in_used = true;
     }
     int sent = 0, chunk = 0;            // calls whose activations have been submitted, and in how many chunks
     size_t sent_off = 0, sent_d_off = 0;
@@ -1619,6 +1641,7 @@ extern "C" int hfrk_skinny_gemm_fp8_host_batch(const hfrk_host_call* calls, int 
         cudaEvent_t e = next_event();
         HFRK_CUDA_TRY(cudaEventRecord(e, res->in_stream));
         HFRK_CUDA_TRY(cudaStreamWaitEvent(res->out_stream, e, 0));
+        join.out_used = true;
     }
 
     // Results leave on the outbound stream in groups of at least an eighth of them and kBatchMergeBytes: each
@@ -1638,6 +1661,7 @@ extern "C" int hfrk_skinny_gemm_fp8_host_batch(const hfrk_host_call* calls, int 
         cudaEvent_t e = next_event();
         HFRK_CUDA_TRY(cudaEventRecord(e, s));
         HFRK_CUDA_TRY(cudaStreamWaitEvent(res->out_stream, e, 0));
+        join.out_used = true;
         size_t off = group_first_off;
         int i = group_first;
         while (i <= last) {
@@ -1706,6 +1730,7 @@ extern "C" int hfrk_skinny_gemm_fp8_host_batch(const hfrk_host_call* calls, int 
     cudaEvent_t done = next_event();
     HFRK_CUDA_TRY(cudaEventRecord(done, res->out_stream));
     HFRK_CUDA_TRY(cudaStreamWaitEvent(s, done, 0));
+    join.complete = true;   // the inbound stream was waited for chunk by chunk
     return HFRK_SUCCESS;
 }
 

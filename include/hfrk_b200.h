@@ -142,7 +142,7 @@ int hfrk_skinny_gemm_fp8_host_async(const void* A_host, const void* W_dev, void*
  * work_dev: device scratch of at least hfrk_host_batch_workspace_bytes(calls, count) bytes; host
  * buffers should be page-locked (pageable ones make the copies synchronous, still correct) and
  * must stay untouched until `stream` has been synchronised. Returns the first failing call's
- * status. No counterpart in the reference, whose callers hold activations in CUDA tensors
+ * status; the calls before it may have been queued, and `stream` then waits for their copies too. No counterpart in the reference, whose callers hold activations in CUDA tensors
  * (hf_rocm_kernels/operators/skinny_gemm/wrapped.py:104-128). */
 typedef struct hfrk_host_call {
     const void* A_host;      /* [m, k] fp8 */

@@ -75,3 +75,39 @@ def test_results_over_inputs_of_later_calls(capi, pinned, count):
         stream.synchronize()
         assert torch.equal(d_host, want.cpu())
     assert capi.device_status(clear=True)[0] == 0
+
+
+@pytest.mark.gpu
+def test_a_batch_that_fails_half_way_is_joined_to_its_stream(capi):
+    """The third call's weight pitch is refused after two calls were queued with their copies: one synchronise of
+    the stream still covers those, and a batch on the same scratch right behind it is not disturbed."""
+    dev = torch.device("cuda:0")
+    m, n, k = 16, 28672, 1024                        # every result is a group of its own
+    gen = torch.Generator().manual_seed(9)
+    scale = torch.tensor([2e-4], device=dev)
+    calls, want = [], []
+    for i in range(6):
+        a = torch.randint(0, 120, (m, k), generator=gen, dtype=torch.uint8)
+        w = torch.randint(0, 120, (n, k), generator=gen, dtype=torch.uint8).view(torch.float8_e4m3fn).to(dev)
+        d_in = torch.randn((m, n), generator=gen).bfloat16().pin_memory()
+        expect = d_in.to(dev)
+        capi.check(capi.skinny_gemm(a.view(torch.float8_e4m3fn).to(dev), w, expect, scale))
+        want.append(expect.cpu())
+        calls.append((a.pin_memory().view(torch.float8_e4m3fn), w, torch.zeros((m, n), dtype=torch.bfloat16).pin_memory(), scale,
+                      True, d_in))
+    batch = capi.HostBatch(calls, dev)
+    stream = torch.cuda.Stream()
+    for _ in range(3):
+        for call in calls:
+            call[2].fill_(0.0)
+        batch.array[2].w_row_stride = k + 8
+        assert batch.queue(stream) == 7              # HFRK_BAD_ALIGNMENT
+        stream.synchronize()
+        assert all(torch.equal(calls[i][2], want[i]) for i in range(2))
+        assert all(int(calls[i][2].count_nonzero()) == 0 for i in range(2, 6))
+        assert batch.queue(stream) == 7
+        batch.array[2].w_row_stride = k
+        capi.check(batch.queue(stream))
+        stream.synchronize()
+        assert all(torch.equal(call[2], w) for call, w in zip(calls, want))
+    assert capi.device_status(clear=True)[0] == 0
