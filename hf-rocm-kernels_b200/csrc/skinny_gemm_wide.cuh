@@ -94,7 +94,7 @@ __device__ __forceinline__ uint4 wide_swiglu_16(const float (&gate)[16], const f
     }
     uint32_t words[4];
     // the fast path encodes e4m3fnuz through twice the scale, which must not overflow
-    if (top <= kSiluFastLimit && inv_act < 1e38f) {
+    if (top <= kSiluFastLimit && fabsf(inv_act) < 1e38f) {
         const float inv_fast = fnuz ? 2.0f * inv_act : inv_act;
         const float2 inv = make_float2(inv_fast, inv_fast);
 #pragma unroll

@@ -60,7 +60,7 @@ __device__ __forceinline__ uint2 swiglu_8(const uint4& gate_raw, const uint4& up
     const float2 top = pair_f32(max_abs(max_abs(g[0] & abs_mask, g[1] & abs_mask, T()),
                                         max_abs(g[2] & abs_mask, g[3] & abs_mask, T()), T()), T());
     // the fast path encodes e4m3fnuz through twice the scale, which must not overflow
-    const bool fast = fmaxf(top.x, top.y) <= kSiluFastLimit && inv_scale < 1e38f;
+    const bool fast = fmaxf(top.x, top.y) <= kSiluFastLimit && fabsf(inv_scale) < 1e38f;
     const float inv_fast = kFnuz ? 2.0f * inv_scale : inv_scale;
     const float2 inv = make_float2(inv_fast, inv_fast);
     uint32_t half_words[4];

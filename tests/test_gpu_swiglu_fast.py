@@ -14,10 +14,10 @@ def _both(gate_up, scale, fp8):
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("fp8", [torch.float8_e4m3fn, torch.float8_e4m3fnuz])
-@pytest.mark.parametrize("scale", [1.0, 0.021, 37.0, 3e-5, 1e-30, 4e-39, 1e-45])
+@pytest.mark.parametrize("scale", [1.0, 0.021, 37.0, 3e-5, 1e-30, 4e-39, 1e-45, -0.021, -4e-39, -1e-45])
 def test_every_16_bit_gate_value(native_build, dtype, fp8, scale):
     """All 65,536 bit patterns as gates (zeros of both signs, subnormals, infinities, NaNs) times four ups; scales
-    down to those whose reciprocal overflows. Vectors hold neighbouring patterns, so that slow and fast
+    of both signs, down to those whose reciprocal overflows. Vectors hold neighbouring patterns, so that slow and fast
     vectors (by their largest gate) both occur."""
     gate = torch.arange(65536, dtype=torch.int32, device="cuda").to(torch.int16).view(dtype).view(8192, 8)
     for up in (1.0, -0.37, 0.0, 250.0):

@@ -174,3 +174,24 @@ def test_mlp_chain_above_16_tokens(capi, dev, tokens, inter):
     graph.replay()
     _ok(capi)
     assert torch.equal(g_out, out)
+
+
+@pytest.mark.parametrize("act,fp8", [(torch.bfloat16, torch.float8_e4m3fn), (torch.float16, torch.float8_e4m3fnuz)])
+@pytest.mark.parametrize("scale", [0.02, -0.02, 4e-39, -4e-39, 1e-45, -1e-45])
+def test_fused_swiglu_under_extreme_scales(capi, dev, act, fp8, scale):
+    """One K block, so that the projection is the same sum in both forms: the same bytes, zero rows (a projection
+    of zero times a scale whose double overflows) among them."""
+    from hf_rocm_kernels import skinny_gemm, swiglu
+
+    m, inter, k = 40, 64, 128
+    a, w, s = _operands(m, 2 * inter, k, fp8, dev)
+    a.view(torch.uint8)[::3] = 0
+    act_scale = torch.tensor([scale], device=dev)
+    gate_up = torch.zeros((m, 2 * inter), dtype=act, device=dev)
+    skinny_gemm(a, w.t(), s, gate_up)
+    expect = swiglu(gate_up, act_scale, out_dtype=fp8, force_scalar=True)
+    out = torch.empty((m, inter), dtype=fp8, device=dev)
+    none = torch.empty((m, 0), dtype=act, device=dev)
+    torch.ops._HFRK_C.gate_up_swiglu(a, w.t(), out, s, act_scale, none, act == torch.bfloat16)
+    _ok(capi)
+    assert torch.equal(out.view(torch.uint8), expect.view(torch.uint8))
