@@ -249,18 +249,26 @@ int make_plan(const DeviceModel& dm, int m, int n, int k, int split_req, int sta
     const int stage_bytes = kWStageBytes + m_pad * kBlockK;
     const int two_per_sm = 2 * dm.sms;
 
-    // all clusters of (split, stages) resident at once on this device, with room for `spare` more?
+    // all clusters of (split, stages) resident at once on this device, with room for one more, or for `spare` more
+    // where up to 16 tokens put three CTAs on an SM?
     auto resident = [&](int split, int stages, int spare) {
         const int smem = plan_smem_bytes(m, m_pad, split, stages);
         if (smem > kSmemLimit) return false;
         const int per_sm = ctas_per_sm(smem) < max_per_sm ? ctas_per_sm(smem) : max_per_sm;
-        // At the exact capacity a straggler of the previous grid keeps the last cluster out: one stays free. Shapes
-        // of the rule that put three CTAs on an SM (up to 16 tokens) leave two: with a single one the last cluster
-        // still starts late there (10336 x 6992 as 81 clusters of 5 where 82 fit: 17.0 us, 14.5 with clusters
-        // of 4; 3792 x 11792 as 30 clusters of 12 where 31 fit: 11.6 us, 10.0 with clusters of 9).
-        if (spare > 1 && (m_pad != 16 || per_sm < 3)) spare = 1;
-        return per_sm >= 1 && tiles + spare <= dm.capacity[split][per_sm];
+        // At the exact capacity a straggler of the previous grid keeps the last cluster out: one stays free.
+        if (per_sm < 1) return false;
+        return tiles + (m_pad == 16 && per_sm == 3 ? spare : 1) <= dm.capacity[split][per_sm];
     };
+
+    // Clusters that the rule leaves free at three CTAs per SM. With one the last cluster may still start late; with two
+    // the grid may have to go down to a smaller split. Grids that fill the capacity but for one cluster, as they are
+    // against the next smaller split, K of 2048 to 12288 at 1, 8 and 16 tokens:
+    //   * clusters of 11 to 15: 5 to 55 % slower (3792 x 11792 as 30 clusters of 12 where 31 fit: 11.6 us, 10.0 as 9);
+    //   * of 5: 5 % faster or 20 % slower (10336 x 6992 as 81 where 82 fit: 17.0 us, 14.5 as 4);
+    //   * of 6 to 10 with up to four K blocks per CTA 3 to 16 % slower, with more up to 7 % faster (7000 x 7168 9.8 us
+    //     as 55 clusters of 7 where 56 fit, 10.5 as 6);
+    //   * of up to 4: faster (13144 x 4096 as 103 clusters of 4 where 104 fit: 9.9 us, 10.9 as 3).
+    auto spare_clusters = [&](int split) { return split <= 4 || (split > 5 && split <= 10 && nkb > 4 * split) ? 1 : 2; };
 
     TuneValue tuned;
     if (split_req == 0 && stages_req == 0 && tile_rows_req == 0) {
@@ -303,7 +311,7 @@ int make_plan(const DeviceModel& dm, int m, int n, int k, int split_req, int sta
                 for (int s = kMaxSplit; s >= 2; --s) {
                     const bool few = m_pad == 16 && s <= nkb && tiles * s <= dm.sms;
                     if (nkb / s < 2 && !few) continue;
-                    if (!resident(s, ring, 2)) continue;
+                    if (!resident(s, ring, spare_clusters(s))) continue;
                     const int ctas = tiles * s;
                     bool better;
                     if (m_pad > 16) {

@@ -47,3 +47,19 @@ def test_one_cluster_stays_free_at_two_ctas_per_sm(capi, spare, split):
     """Two CTAs per SM (nothing larger than 5 fits, nothing at all at three per SM): 40 tiles need room for 41."""
     none = {s: (0, 0, 0) for s in (2, 3, *range(6, 17))}
     assert _plan(capi, 16, 5120, 9600, {**none, 4: (37, 74, 0), 5: (20, 40 + spare, 0)})["split_k"] == split
+
+
+# (tiles, K blocks, split that needs all but one cluster, the next smaller one that fits with two to spare)
+@pytest.mark.parametrize("tiles,k,split,smaller,two", [
+    (30, 4096, 12, 10, True), (23, 12288, 15, 13, True),           # clusters of 11 and more
+    (55, 2048, 7, 6, True), (47, 4096, 8, 7, True),                # 6 to 10, up to four K blocks per CTA
+    (55, 4096, 7, 6, False), (47, 12288, 8, 7, False),             # more of them
+    (103, 4096, 4, 3, False), (103, 12288, 4, 3, False)])          # up to 4
+@pytest.mark.parametrize("m", [1, 16])
+def test_how_many_clusters_stay_free(capi, m, tiles, k, split, smaller, two):
+    for spare in (1, 2):
+        capacity = {s: 0 for s in range(split + 1, 17)}
+        capacity.update({s: tiles for s in range(smaller + 1, split)})     # full: never taken
+        capacity.update({split: tiles + spare, smaller: 4 * tiles})
+        got = _plan(capi, m, tiles * 128, k, capacity)["split_k"]
+        assert got == (split if spare == 2 or not two else smaller)
