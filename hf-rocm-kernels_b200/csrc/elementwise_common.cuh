@@ -49,8 +49,8 @@ __device__ __forceinline__ float silu_f32(float x) { return x / (1.0f + expf(-x)
 // quotient by an approximate reciprocal is corrected once with its exact remainder (Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000 processor", 1990), two values per
 // instruction. The limit keeps 1 + e^-x far from overflow, where the remainder would be NaN. The
-// reciprocal is taken negative so that a zero keeps its sign. Equal to silu_f32 after the conversion to
-// fp8 for every fp16 and bf16 value (tests/test_gpu_swiglu_fast.py).
+// reciprocal is taken negative so that a zero keeps its sign. Not correctly rounded for every fp32 argument,
+// but the same bits as silu_f32 for all 77,636 fp16 and bf16 values within the limit (compared one by one).
 constexpr float kSiluFastLimit = 80.0f;
 __device__ __forceinline__ float2 silu_f32x2(float2 minus_x) {
     const float2 one = make_float2(1.0f, 1.0f);

@@ -307,10 +307,16 @@ int make_plan(const DeviceModel& dm, int m, int n, int k, int split_req, int sta
             for (int choice = m_pad > 16 ? 0 : 1; choice < 3; ++choice) {
                 const int ring = stages_req != 0 ? stages_req : ring_choices[choice];
                 // Up to 16 tokens one K block per CTA is enough while the CTAs do not fill the SMs (1104 x 1104:
-                // 3.4 us with clusters of 4, 2.9 with clusters of 9).
+                // 3.4 us with clusters of 4, 2.9 with clusters of 9), and so are one or two, where the split that
+                // gives every CTA two has a CTA with three (848 x 2368: 3.4 us with 9, 3.2 with 16). A larger split
+                // whose longest range is two as well only adds partials (1400 x 2256: 3.4 us with 9, 3.7 with 13).
                 for (int s = kMaxSplit; s >= 2; --s) {
-                    const bool few = m_pad == 16 && s <= nkb && tiles * s <= dm.sms;
-                    if (nkb / s < 2 && !few) continue;
+                    if (nkb / s < 2) {
+                        const bool few = m_pad == 16 && s <= nkb && tiles * s <= dm.sms;
+                        const bool same_range = s < nkb && nkb % 2 == 0 && nkb / 2 <= kMaxSplit &&
+                                                resident(nkb / 2, ring, spare_clusters(nkb / 2));
+                        if (!few || same_range) continue;
+                    }
                     if (!resident(s, ring, spare_clusters(s))) continue;
                     const int ctas = tiles * s;
                     bool better;

@@ -1,0 +1,96 @@
+"""Which kernel and which launch shape a call takes (CPU only, capacities of an imagined chip)."""
+import pytest
+
+
+@pytest.fixture(scope="module")
+def capi(native_build):
+    from hf_rocm_kernels import _capi
+
+    return _capi
+
+
+@pytest.fixture(autouse=True)
+def chip(capi):
+    """A chip whose GPCs hold 85 % of the clusters that the SM count allows."""
+    table = [[0, 0, 0, 0]] + [[0] + [148 * p // s * (100 if s == 1 else 85) // 100 for p in (1, 2, 3)] for s in range(1, 17)]
+    capi.override_device_model(148, table)
+    yield
+    capi.override_device_model(capacity=None)
+
+
+CLUSTER, STREAMK, WIDE = 1, 2, 3
+
+
+@pytest.mark.parametrize("n,k", [(4096, 4096), (28672, 4096), (17, 128), (8192, 28672)])
+def test_more_than_64_tokens_run_wide_and_up_to_16_do_not(capi, n, k):
+    for m in (1, 16):
+        assert capi.launch_info(m, n, k)["kernel"] == CLUSTER
+    for m in (65, 128, 129, 256, 257, 1000):
+        info = capi.launch_info(m, n, k)
+        assert info["kernel"] == WIDE
+        launches = -(-m // 256)
+        assert 0 <= info["m_pad"] - -(-m // launches) < 16     # the tokens of one launch, shared out evenly
+
+
+def test_explicit_and_tuned_calls_stay_on_the_kernel_they_name(capi):
+    for m in (65, 130, 256):
+        assert capi.launch_info(m, 2000, 4096, split_k=3)["kernel"] == CLUSTER
+        assert capi.launch_info(m, 2000, 4096, num_stages=4)["kernel"] == CLUSTER
+        assert capi.launch_info(m, 2000, 4096, kernel=CLUSTER)["kernel"] == CLUSTER
+        assert capi.launch_info(m, 2000, 4096, kernel=STREAMK)["kernel"] == STREAMK
+    capi.lib.hfrk_tuning_set(64, 2000, 4096, 2, 3)
+    try:
+        info = capi.launch_info(130, 2000, 4096)
+        assert (info["kernel"], info["split_k"], info["num_stages"]) == (CLUSTER, 2, 3)
+        assert capi.launch_info(130, 2016, 4096)["kernel"] == WIDE
+        assert capi.launch_info(130, 2000, 4096, kernel=WIDE)["kernel"] == WIDE
+    finally:
+        capi.lib.hfrk_tuning_clear()
+    assert capi.launch_info(130, 2000, 4096)["kernel"] == WIDE
+
+
+@pytest.mark.parametrize("m,kernel", [(1, CLUSTER), (16, CLUSTER), (17, WIDE), (64, WIDE), (65, WIDE), (300, WIDE)])
+def test_swiglu_form(capi, m, kernel):
+    assert capi.launch_info(m, 2048, 1024, swiglu=True)["kernel"] == kernel
+
+
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("m", [1, 17, 64, 128, 129, 200, 256])
+def test_every_pinned_shape_keeps_its_bounds(capi, m, swiglu):
+    """Ring, receive buffer and TMEM of every shape that the planner lets through, by the layouts of the kernel."""
+    halves = 2 if m > 128 else 1
+    rows = -(-(-(-m // halves)) // 8) * 8 * halves
+    step = 32 if swiglu else 16
+    for split in range(1, 9):
+        for tile in range(32, 257, step):
+            for stages in (2, 8):
+                for per_sm in (1, 2):
+                    out = (capi.ctypes.c_int * 8)()
+                    rc = capi.lib.hfrk_gemm_launch_info(m, 2080, 2064, int(swiglu), WIDE, split, tile, stages, per_sm, out)
+                    if rc != 0:
+                        assert rc == 6
+                        continue
+                    kernel, got_split, got_stages, ctas, smem, m_pad, k_blocks, rows_w = list(out)
+                    assert (kernel, got_split, m_pad, k_blocks, rows_w) == (WIDE, split, rows, 17, tile)
+                    assert 2 <= got_stages <= stages and ctas == -(-2080 // tile) * split
+                    ring = got_stages * (halves * 16384 + tile * 128)
+                    groups = tile // step
+                    assert groups >= split
+                    if split > 1:
+                        assert split * -(-groups // split) * step * (rows + 1) * 4 <= ring
+                        assert ctas // split <= 148 * per_sm // split * 85 // 100
+                    else:
+                        assert 8 * 32 * 36 * 4 <= ring
+                    columns = halves * max(32, 1 << (tile - 1).bit_length())
+                    assert 1024 + ring < smem <= 227 * 1024 and per_sm * (smem + 1024) <= 228 * 1024
+                    assert columns * per_sm <= 512 and (smem + 1024) * 512 >= columns * 228 * 1024 * 0.999
+
+
+def test_bad_queries(capi):
+    out = (capi.ctypes.c_int * 8)()
+    for args in ((0, 128, 128, 0, 0), (16, 128, 128, 0, 4), (16, 127, 128, 1, 0), (16, 128, 128, 1, 1), (300, 128, 128, 0, -1)):
+        assert capi.lib.hfrk_gemm_launch_info(*args, 0, 0, 0, 0, out) == 6
+    assert capi.lib.hfrk_gemm_launch_info(200, 128, 128, 0, WIDE, 9, 0, 0, 0, out) == 6       # more than eight CTAs per cluster
+    assert capi.lib.hfrk_gemm_launch_info(200, 128, 128, 0, WIDE, 2, 0, 0, 0, out) == 6       # more than the K blocks
+    assert capi.lib.hfrk_gemm_launch_info(200, 128, 128, 0, WIDE, 0, 40, 0, 0, out) == 6      # no multiple of 16
+    assert capi.lib.hfrk_wide_gemm_fp8(0, 0, 0, 0, 0, 16, 128, 128, 128, 0, 0, 1, 0, 0, 0, 0, 0, 0, 0) == 6
