@@ -1,5 +1,5 @@
-// FP8 GEMM for the larger decode batches (65 .. 256 tokens per launch) on B200 (sm_100a), plain and
-// with swiglu in the epilogue.
+// FP8 GEMM for the larger decode batches (above 64 tokens, and 17 to 64 by a rule; up to 256 per launch) on
+// B200 (sm_100a), plain and with swiglu in the epilogue.
 //
 // What bounds it: up to 256 tokens the product still needs only one pass over W, so the floor is the
 // larger of N*K bytes of HBM and 2*M*N*K operations of the tensor cores (they meet near 250 tokens).
@@ -142,17 +142,40 @@ __device__ __forceinline__ bool wide_vec_ok(const WideParams& p, int token, int 
     return token < p.m && col + 8 <= p.n && ((reinterpret_cast<uintptr_t>(p.d) + idx * out_bytes<DT>()) & 15u) == 0;
 }
 
+// D_in of a piece. Where rows of D are not 16-byte aligned its elements are read one by one, or in pairs, all
+// of them before anything is stored: a load behind a store has to wait for it, and as eight such pairs per
+// piece 14933 x 1024 at 29 tokens took 40 us (9.9 us with the loads ahead, 8.4 us storing).
 template <int DT>
 __device__ __forceinline__ Raw8<DT> wide_load_din(const WideParams& p, int token, int col, bool wanted) {
+    constexpr int kWords = DT == HFRK_F32 ? 8 : 4;
+    uint32_t w[kWords];
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) w[i] = 0u;
+    if (wanted && p.accumulate && token < p.m) {
+        const uint8_t* const src = static_cast<const uint8_t*>(p.d) + (static_cast<size_t>(token) * p.n + col) * out_bytes<DT>();
+        const int left = p.n - col;
+        if (wide_vec_ok<DT>(p, token, col)) {
+#pragma unroll
+            for (int i = 0; i < kWords / 4; ++i) {
+                const uint4 q = reinterpret_cast<const uint4*>(src)[i];
+                w[4 * i] = q.x; w[4 * i + 1] = q.y; w[4 * i + 2] = q.z; w[4 * i + 3] = q.w;
+            }
+        } else if constexpr (DT == HFRK_F32) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i < left) w[i] = reinterpret_cast<const uint32_t*>(src)[i];
+        } else if ((reinterpret_cast<uintptr_t>(src) & 3u) == 0 && left >= 8) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i] = reinterpret_cast<const uint32_t*>(src)[i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i < left) w[i >> 1] |= static_cast<uint32_t>(reinterpret_cast<const uint16_t*>(src)[i]) << (16 * (i & 1));
+        }
+    }
     Raw8<DT> r;
 #pragma unroll
-    for (int i = 0; i < (DT == HFRK_F32 ? 2 : 1); ++i) r.q[i] = make_uint4(0, 0, 0, 0);
-    if (wanted && p.accumulate && wide_vec_ok<DT>(p, token, col)) {
-        const size_t idx = static_cast<size_t>(token) * p.n + col;
-        const uint4* src = reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(p.d) + idx * out_bytes<DT>());
-#pragma unroll
-        for (int i = 0; i < (DT == HFRK_F32 ? 2 : 1); ++i) r.q[i] = src[i];
-    }
+    for (int i = 0; i < kWords / 4; ++i) r.q[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
     return r;
 }
 
@@ -161,44 +184,43 @@ template <int DT>
 __device__ __forceinline__ void wide_store_piece(const WideParams& p, int token, int col, float scale, const float (&x)[8],
                                                  const Raw8<DT>& din) {
     if (token >= p.m || col >= p.n) return;
-    const size_t idx = static_cast<size_t>(token) * p.n + col;
-    if (wide_vec_ok<DT>(p, token, col)) {
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.d) + idx * out_bytes<DT>());
+    constexpr int kWords = DT == HFRK_F32 ? 8 : 4;
+    uint32_t in[kWords], out[kWords];
+#pragma unroll
+    for (int i = 0; i < kWords / 4; ++i) {
+        in[4 * i] = din.q[i].x; in[4 * i + 1] = din.q[i].y; in[4 * i + 2] = din.q[i].z; in[4 * i + 3] = din.q[i].w;
+    }
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) {
         if constexpr (DT == HFRK_F32) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                dst[i] = make_uint4(__float_as_uint(fmaf(x[4 * i], scale, __uint_as_float(din.q[i].x))),
-                                    __float_as_uint(fmaf(x[4 * i + 1], scale, __uint_as_float(din.q[i].y))),
-                                    __float_as_uint(fmaf(x[4 * i + 2], scale, __uint_as_float(din.q[i].z))),
-                                    __float_as_uint(fmaf(x[4 * i + 3], scale, __uint_as_float(din.q[i].w))));
-            }
+            out[i] = __float_as_uint(fmaf(x[i], scale, __uint_as_float(in[i])));
+        } else if constexpr (DT == HFRK_BF16) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&in[i]));
+            const __nv_bfloat162 h = __floats2bfloat162_rn(fmaf(x[2 * i], scale, f.x), fmaf(x[2 * i + 1], scale, f.y));
+            out[i] = *reinterpret_cast<const uint32_t*>(&h);
         } else {
-            const uint32_t in[4] = {din.q[0].x, din.q[0].y, din.q[0].z, din.q[0].w};
-            uint32_t out[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                float2 f;
-                if constexpr (DT == HFRK_BF16) {
-                    f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&in[i]));
-                    const __nv_bfloat162 h =
-                        __floats2bfloat162_rn(fmaf(x[2 * i], scale, f.x), fmaf(x[2 * i + 1], scale, f.y));
-                    out[i] = *reinterpret_cast<const uint32_t*>(&h);
-                } else {
-                    f = __half22float2(*reinterpret_cast<const __half2*>(&in[i]));
-                    const __half2 h = __floats2half2_rn(fmaf(x[2 * i], scale, f.x), fmaf(x[2 * i + 1], scale, f.y));
-                    out[i] = *reinterpret_cast<const uint32_t*>(&h);
-                }
-            }
-            dst[0] = make_uint4(out[0], out[1], out[2], out[3]);
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&in[i]));
+            const __half2 h = __floats2half2_rn(fmaf(x[2 * i], scale, f.x), fmaf(x[2 * i + 1], scale, f.y));
+            out[i] = *reinterpret_cast<const uint32_t*>(&h);
         }
+    }
+    uint8_t* const dst = static_cast<uint8_t*>(p.d) + (static_cast<size_t>(token) * p.n + col) * out_bytes<DT>();
+    const int left = p.n - col;
+    if (wide_vec_ok<DT>(p, token, col)) {
+#pragma unroll
+        for (int i = 0; i < kWords / 4; ++i)
+            reinterpret_cast<uint4*>(dst)[i] = make_uint4(out[4 * i], out[4 * i + 1], out[4 * i + 2], out[4 * i + 3]);
+    } else if constexpr (DT == HFRK_F32) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (i < left) reinterpret_cast<uint32_t*>(dst)[i] = out[i];
+    } else if ((reinterpret_cast<uintptr_t>(dst) & 3u) == 0 && left >= 8) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) reinterpret_cast<uint32_t*>(dst)[i] = out[i];
     } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            if (col + j < p.n) {
-                const float d0 = p.accumulate ? load1<DT>(p.d, idx + j) : 0.0f;
-                store1<DT>(p.d, idx + j, fmaf(x[j], scale, d0));
-            }
-        }
+        for (int i = 0; i < 8; ++i)
+            if (i < left) reinterpret_cast<uint16_t*>(dst)[i] = static_cast<uint16_t>(out[i >> 1] >> (16 * (i & 1)));
     }
 }
 
@@ -346,12 +368,15 @@ __device__ __forceinline__ void wide_epilogue_owner(const WideParams& p, const f
     const int rows = p.halves * p.rows_half, pieces = 2 * own > 0 ? 2 * own : 1, items = own > 0 ? rows * pieces : 0;
     const int n0 = blockIdx.x * p.tile_n + lo * 16;
     Raw8<DT> din[kAhead];
+    auto load_ahead = [&](int base) {
 #pragma unroll
-    for (int i = 0; i < kAhead; ++i) {
-        const int item = static_cast<int>(threadIdx.x) + i * kStep;
-        const int row = item / pieces;
-        din[i] = wide_load_din<DT>(p, row, n0 + (item - row * pieces) * 8, item < items);
-    }
+        for (int i = 0; i < kAhead; ++i) {
+            const int item = base + i * kStep;
+            const int row = item / pieces;
+            din[i] = wide_load_din<DT>(p, row, n0 + (item - row * pieces) * 8, item < items);
+        }
+    };
+    load_ahead(threadIdx.x);
     const bool ok = wait_accum();
     send();
     if (own == 0) return;
@@ -359,12 +384,12 @@ __device__ __forceinline__ void wide_epilogue_owner(const WideParams& p, const f
     const bool landed = mbar_wait_bounded(recv_bar, 0u, &own_abort, kRoleEpilogue);
     if (!landed || !ok) return;
     for (int base = threadIdx.x; base < items; base += kAhead * kStep) {
+        if (base != static_cast<int>(threadIdx.x)) load_ahead(base);
 #pragma unroll
         for (int i = 0; i < kAhead; ++i) {
             const int item = base + i * kStep;
             if (item >= items) break;
             const int row = item / pieces, piece = item - row * pieces;
-            if (base != static_cast<int>(threadIdx.x)) din[i] = wide_load_din<DT>(p, row, n0 + piece * 8, true);
             float x[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
             for (int s = 0; s < p.split; ++s) {
                 const uint32_t at = wide_recv_index(s, own, piece >> 1, 1, 0, (piece & 1) * 2, rows + 1, row);
