@@ -744,6 +744,10 @@ int make_wide_plan(const DeviceModel& dm, int m, int n, int k, bool swiglu, cons
 //     reduction runs past its registers, D_in late: 6144 x 4096 at 64 tokens 9.9 us against 12.3,
 //     10240 x 8192 19.2 against 29.1, 8192 x 8192 16.2 against 17.7; overwriting D, the two are even.
 // Elsewhere up to 64 tokens the skinny kernel is ahead (by 1 to 3 us, most at the fewest tokens).
+bool pins_launch_shape(int variant, int split_req, int ctas_per_sm, int stages_req) {
+    return variant != HFRK_VARIANT_AUTO || split_req != 0 || ctas_per_sm != 0 || stages_req != 0;
+}
+
 bool use_wide_kernel(const DeviceModel& dm, int m, int n, int k, bool explicit_shape) {
     if (explicit_shape || m <= 16) return false;
     TuneValue tuned;
@@ -755,21 +759,24 @@ bool use_wide_kernel(const DeviceModel& dm, int m, int n, int k, bool explicit_s
     return plan.split == 1 ? plan.ctas > ctas_per_sm(plan.smem_bytes) * dm.sms : (1 << plan.rows_log2) > kOwned;
 }
 
+int wide_tokens_per_launch(int m) {
+    const int chunks = (m - 1) / kWideMaxTokens + 1;
+    return (m - 1) / chunks + 1;
+}
+
 // One launch per 256 tokens, the tokens shared out evenly. The caller has validated the arguments.
 // `p` carries the outputs (d or act_out / zero_ptr of the whole call) and the scalars.
 template <bool kSwiglu>
-int launch_wide(const void* A, const void* W, int m, int n, int k, int64_t w_row_stride, WideParams p, int use_pdl,
-                cudaStream_t stream) {
+int launch_wide(const void* A, const void* W, int m, int n, int k, int64_t w_row_stride, WideParams p, const WideReq& req,
+                int use_pdl, cudaStream_t stream) {
     const DeviceModel dm = device_model(stream);
-    const int chunks = (m + kWideMaxTokens - 1) / kWideMaxTokens;
-    const int m_step = (m + chunks - 1) / chunks;
+    const int m_step = wide_tokens_per_launch(m);
     uint8_t* const d = static_cast<uint8_t*>(p.d);
     uint8_t* const act_out = p.act_out;
     const size_t out_elem = p.d_dtype == HFRK_F32 ? 4 : 2;
     for (int m0 = 0; m0 < m; m0 += m_step) {
         const int mc = m - m0 < m_step ? m - m0 : m_step;
         WidePlan plan;
-        const WideReq req;
         int rc = make_wide_plan(dm, mc, n, k, kSwiglu, req, &plan);
         if (rc != HFRK_SUCCESS) return rc;
         const int tile_rows = kSwiglu ? plan.tile_n / 2 : plan.tile_n;
@@ -824,6 +831,17 @@ int launch_wide(const void* A, const void* W, int m, int n, int k, int64_t w_row
     return HFRK_SUCCESS;
 }
 
+WideParams wide_params(void* D, const float* scale_dev, int a_kind, int w_kind, int d_dtype, int accumulate) {
+    WideParams p;
+    memset(&p, 0, sizeof(p));
+    p.d = D;
+    p.scale = scale_dev;
+    p.kind_factor = (a_kind == HFRK_E4M3FNUZ ? 0.5f : 1.0f) * (w_kind == HFRK_E4M3FNUZ ? 0.5f : 1.0f);
+    p.d_dtype = d_dtype;
+    p.accumulate = accumulate ? 1 : 0;
+    return p;
+}
+
 int launch_gemm(const void* A, const void* W, void* D, const float* scale_dev, int m, int n, int k,
                 int64_t w_row_stride, int a_kind, int w_kind, int d_dtype, int accumulate, int variant,
                 int split_req, int ctas_per_sm, int stages_req, int use_pdl, cudaStream_t stream,
@@ -834,8 +852,8 @@ int launch_gemm(const void* A, const void* W, void* D, const float* scale_dev, i
     rc = prepare_device_once();
     if (rc != HFRK_SUCCESS) return rc;
     if (variant < HFRK_VARIANT_AUTO || variant > HFRK_VARIANT_STREAMK) return HFRK_INVALID_CONFIG;
-    const bool explicit_shape = variant != HFRK_VARIANT_AUTO || split_req != 0 || ctas_per_sm != 0 || stages_req != 0 ||
-                                tile_rows_req != 0 || stamps != nullptr;
+    const bool explicit_shape = pins_launch_shape(variant, split_req, ctas_per_sm, stages_req) || tile_rows_req != 0 ||
+                                stamps != nullptr;
     if (variant == HFRK_VARIANT_AUTO) variant = HFRK_VARIANT_CLUSTER;
     if (rowpar != nullptr && variant != HFRK_VARIANT_CLUSTER) return HFRK_INVALID_CONFIG;
     if (variant == HFRK_VARIANT_STREAMK) {
@@ -844,14 +862,8 @@ int launch_gemm(const void* A, const void* W, void* D, const float* scale_dev, i
     }
 
     if (use_wide_kernel(device_model(stream), m, n, k, rowpar != nullptr || explicit_shape)) {
-        WideParams p;
-        memset(&p, 0, sizeof(p));
-        p.d = D;
-        p.scale = scale_dev;
-        p.kind_factor = (a_kind == HFRK_E4M3FNUZ ? 0.5f : 1.0f) * (w_kind == HFRK_E4M3FNUZ ? 0.5f : 1.0f);
-        p.d_dtype = d_dtype;
-        p.accumulate = accumulate ? 1 : 0;
-        return launch_wide<false>(A, W, m, n, k, w_row_stride, p, use_pdl, stream);
+        return launch_wide<false>(A, W, m, n, k, w_row_stride, wide_params(D, scale_dev, a_kind, w_kind, d_dtype, accumulate),
+                                  WideReq(), use_pdl, stream);
     }
 
     const size_t out_elem = d_dtype == HFRK_F32 ? 4 : 2;
@@ -949,7 +961,7 @@ int launch_gemm(const void* A, const void* W, void* D, const float* scale_dev, i
 int launch_gemm_swiglu(const void* A, const void* W, void* act_out, const float* scale_dev,
                        const float* act_scale_dev, void* next_buffer, int m, int inter, int k, int64_t w_row_stride,
                        int a_kind, int w_kind, int mid_dtype, int out_kind, int64_t buffer_cols, int split_req,
-                       int use_pdl, bool any_tokens, cudaStream_t stream) {
+                       int use_pdl, bool any_tokens, cudaStream_t stream, const WideReq* wide_req = nullptr) {
     if (A == nullptr || W == nullptr || act_out == nullptr || scale_dev == nullptr || act_scale_dev == nullptr)
         return HFRK_INVALID_CONFIG;
     if (m <= 0 || inter <= 0 || k <= 0 || buffer_cols < 0) return HFRK_INVALID_CONFIG;
@@ -968,20 +980,17 @@ int launch_gemm_swiglu(const void* A, const void* W, void* act_out, const float*
     int rc = prepare_device_once();
     if (rc != HFRK_SUCCESS) return rc;
 
-    if (m > 16) {
+    if (m > 16 || wide_req != nullptr) {
         if (inter > INT32_MAX / 2) return HFRK_INVALID_CONFIG;
-        WideParams wp;
-        memset(&wp, 0, sizeof(wp));
-        wp.scale = scale_dev;
-        wp.kind_factor = (a_kind == HFRK_E4M3FNUZ ? 0.5f : 1.0f) * (w_kind == HFRK_E4M3FNUZ ? 0.5f : 1.0f);
-        wp.d_dtype = mid_dtype;
+        WideParams wp = wide_params(nullptr, scale_dev, a_kind, w_kind, mid_dtype, /*accumulate=*/0);
         wp.act_out = static_cast<uint8_t*>(act_out);
         wp.act_scale = act_scale_dev;
         wp.act_cols = inter;
         wp.act_fnuz = out_kind == HFRK_E4M3FNUZ ? 1 : 0;
         wp.zero_ptr = static_cast<uint8_t*>(next_buffer);
         wp.zero_bytes = zero_bytes;
-        return launch_wide<true>(A, W, m, 2 * inter, k, w_row_stride, wp, use_pdl, stream);
+        return launch_wide<true>(A, W, m, 2 * inter, k, w_row_stride, wp, wide_req != nullptr ? *wide_req : WideReq(), use_pdl,
+                                 stream);
     }
 
     CUtensorMap tmap_w, tmap_a;
@@ -1332,6 +1341,32 @@ extern "C" int hfrk_gate_up_swiglu_fp8(const void* A, const void* W_gate_up, voi
     return hfrk::launch_gemm_swiglu(A, W_gate_up, act_out, scale_dev, act_scale_dev, next_buffer, m, inter, k,
                                     w_row_stride, a_kind, w_kind, mid_dtype, out_kind, buffer_cols, /*split_req=*/0,
                                     hfrk::default_use_pdl(), /*any_tokens=*/true, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int hfrk_wide_gemm_fp8(const void* A, const void* W, void* D, const float* scale_dev,
+                                  const float* act_scale_dev, int m, int n, int k, int64_t w_row_stride, int a_kind,
+                                  int w_kind, int d_dtype, int accumulate, int out_kind, int split_k, int tile_rows,
+                                  int num_stages, int ctas_per_sm, void* stream) {
+    using namespace hfrk;
+    if (split_k < 0 || tile_rows < 0 || num_stages < 0 || ctas_per_sm < 0) return HFRK_INVALID_CONFIG;
+    WideReq req;
+    req.split = split_k;
+    req.tile_n = tile_rows;
+    req.stages = num_stages;
+    req.per_sm = ctas_per_sm;
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (act_scale_dev != nullptr) {
+        if (n % 2 != 0) return HFRK_INVALID_CONFIG;
+        return launch_gemm_swiglu(A, W, D, scale_dev, act_scale_dev, nullptr, m, n / 2, k, w_row_stride, a_kind, w_kind,
+                                  d_dtype, out_kind, /*buffer_cols=*/0, /*split_req=*/0, default_use_pdl(),
+                                  /*any_tokens=*/true, s, &req);
+    }
+    int rc = validate(A, W, D, scale_dev, m, n, k, w_row_stride, a_kind, w_kind, d_dtype);
+    if (rc != HFRK_SUCCESS) return rc;
+    rc = prepare_device_once();
+    if (rc != HFRK_SUCCESS) return rc;
+    return launch_wide<false>(A, W, m, n, k, w_row_stride, wide_params(D, scale_dev, a_kind, w_kind, d_dtype, accumulate), req,
+                              default_use_pdl(), s);
 }
 
 extern "C" int hfrk_skinny_gemm_fp8_ex(const void* A, const void* W, void* D, const float* scale_dev, int m, int n,
@@ -1745,6 +1780,54 @@ extern "C" int hfrk_skinny_gemm_fp8_host_batch(const hfrk_host_call* calls, int 
     HFRK_CUDA_TRY(cudaEventRecord(done, res->out_stream));
     HFRK_CUDA_TRY(cudaStreamWaitEvent(s, done, 0));
     join.complete = true;   // the inbound stream was waited for chunk by chunk
+    return HFRK_SUCCESS;
+}
+
+extern "C" int hfrk_gemm_launch_info(int m, int n, int k, int form, int kernel, int split_k, int tile_rows,
+                                     int num_stages, int ctas_per_sm, int* out8) {
+    using namespace hfrk;
+    const bool swiglu = form == HFRK_FORM_SWIGLU;
+    if (out8 == nullptr || m <= 0 || n <= 0 || k <= 0 || kernel < HFRK_VARIANT_AUTO || kernel > HFRK_KERNEL_WIDE ||
+        form < HFRK_FORM_ACCUMULATE || form > HFRK_FORM_SWIGLU ||
+        (swiglu && (n % 2 != 0 || (kernel != HFRK_VARIANT_AUTO && kernel != HFRK_KERNEL_WIDE))))
+        return HFRK_INVALID_CONFIG;
+    const DeviceModel dm = device_model(nullptr);
+    bool wide = kernel == HFRK_KERNEL_WIDE;
+    if (kernel == HFRK_VARIANT_AUTO) {
+        wide = swiglu ? m > 16
+                      : use_wide_kernel(dm, m, n, k, pins_launch_shape(kernel, split_k, ctas_per_sm, num_stages) || tile_rows != 0);
+    }
+    if (wide) {
+        WideReq req;
+        if (kernel == HFRK_KERNEL_WIDE) {
+            req.split = split_k;
+            req.tile_n = tile_rows;
+            req.stages = num_stages;
+            req.per_sm = ctas_per_sm;
+        }
+        WidePlan plan;
+        const int rc = make_wide_plan(dm, wide_tokens_per_launch(m), n, k, swiglu, req, &plan);
+        if (rc != HFRK_SUCCESS) return rc;
+        const int out[8] = {HFRK_KERNEL_WIDE, plan.split, plan.stages, plan.tiles * plan.split, plan.smem_bytes,
+                            plan.halves * plan.rows_half, plan.num_kblocks, plan.tile_n};
+        memcpy(out8, out, sizeof(out));
+        return HFRK_SUCCESS;
+    }
+    const int mc = m > kMaxMPad ? kMaxMPad : m;
+    if (kernel == HFRK_VARIANT_STREAMK) {
+        SkPlan plan;
+        const int rc = make_sk_plan(mc, n, k, ctas_per_sm, num_stages, &plan);
+        if (rc != HFRK_SUCCESS) return rc;
+        const int out[8] = {HFRK_VARIANT_STREAMK, 0, plan.stages, plan.grid, plan.smem_bytes, plan.m_pad, plan.nkb, kTileN};
+        memcpy(out8, out, sizeof(out));
+        return HFRK_SUCCESS;
+    }
+    Plan plan;
+    const int rc = make_plan(dm, mc, n, k, split_k, num_stages, &plan, swiglu ? kAutoTileRowsOff : tile_rows);
+    if (rc != HFRK_SUCCESS) return rc;
+    const int out[8] = {HFRK_VARIANT_CLUSTER, plan.split, plan.stages, plan.ctas, plan.smem_bytes, plan.m_pad, plan.num_kblocks,
+                        plan.tile_rows};
+    memcpy(out8, out, sizeof(out));
     return HFRK_SUCCESS;
 }
 

@@ -35,7 +35,8 @@ EXPORTED_SYMBOLS = (
     "hfrk_skinny_gemm_fp8_noalloc", "hfrk_max_active_clusters", "hfrk_tuning_set", "hfrk_tuning_clear",
     "hfrk_swiglu_fp8", "hfrk_residual_rms", "hfrk_rowpar_set_mode",
     "hfrk_skinny_gemm_fp8_swiglu", "hfrk_gate_up_swiglu_fp8", "hfrk_skinny_gemm_fp8_host_async",
-    "hfrk_tuning_set_ex", "hfrk_host_batch_inputs_first", "hfrk_rowpar_set_wait_ms", "hfrk_device_model_get", "hfrk_device_model_override",
+    "hfrk_tuning_set_ex", "hfrk_host_batch_inputs_first", "hfrk_gemm_launch_info",
+    "hfrk_wide_gemm_fp8", "hfrk_rowpar_set_wait_ms", "hfrk_device_model_get", "hfrk_device_model_override",
 )
 
 
@@ -103,6 +104,10 @@ def _load() -> ctypes.CDLL:
     lib.hfrk_skinny_gemm_fp8_swiglu.restype = i32
     lib.hfrk_gate_up_swiglu_fp8.argtypes = lib.hfrk_skinny_gemm_fp8_swiglu.argtypes
     lib.hfrk_gate_up_swiglu_fp8.restype = i32
+    lib.hfrk_gemm_launch_info.argtypes = [i32] * 9 + [ctypes.POINTER(i32)]
+    lib.hfrk_gemm_launch_info.restype = i32
+    lib.hfrk_wide_gemm_fp8.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i64] + [i32] * 9 + [vp]
+    lib.hfrk_wide_gemm_fp8.restype = i32
     lib.hfrk_last_error.restype = ctypes.c_char_p
     for name in ("hfrk_skinny_gemm_fp8", "hfrk_skinny_gemm_fp8_ex", "hfrk_skinny_gemm_fp8_host",
                  "hfrk_skinny_gemm_fp8_simt", "hfrk_skinny_gemm_plan", "hfrk_device_status", "hfrk_version"):
@@ -334,6 +339,36 @@ def plan(m: int, n: int, k: int, variant: int = VARIANT_AUTO, split_k: int = 0, 
     check(lib.hfrk_skinny_gemm_plan(m, n, k, variant, split_k, ctas_per_sm, out))
     keys = ("variant", "split_k", "num_stages", "ctas", "smem_bytes", "m_pad", "k_blocks", "tiles")
     return dict(zip(keys, list(out)))
+
+
+KERNEL_WIDE = 3
+
+
+FORM_ACCUMULATE, FORM_STORE, FORM_SWIGLU = 0, 1, 2
+
+
+def launch_info(m: int, n: int, k: int, form: int = FORM_ACCUMULATE, kernel: int = VARIANT_AUTO, split_k: int = 0,
+                tile_rows: int = 0, num_stages: int = 0, ctas_per_sm: int = 0) -> dict:
+    """``hfrk_gemm_launch_info``: the kernel and the launch shape that a call takes (``n`` = 2 * inter for swiglu)."""
+    out = (ctypes.c_int * 8)()
+    check(lib.hfrk_gemm_launch_info(m, n, k, form, kernel, split_k, tile_rows, num_stages, ctas_per_sm, out))
+    keys = ("kernel", "split_k", "num_stages", "ctas", "smem_bytes", "m_pad", "k_blocks", "tile_rows")
+    return dict(zip(keys, list(out)))
+
+
+def wide_gemm(a, w, d, scale, act_scale=None, accumulate=True, mid_dtype=torch.bfloat16, split_k=0, tile_rows=0,
+              num_stages=0, ctas_per_sm=0, stream=None) -> int:
+    """``hfrk_wide_gemm_fp8`` on torch CUDA tensors; with ``act_scale`` ``d`` is the fp8 [M, N / 2] result of swiglu."""
+    m, k = a.shape
+    n = w.shape[0]
+    assert w.shape[1] == k and w.stride(1) == 1 and a.is_contiguous() and d.is_contiguous()
+    assert tuple(d.shape) == (m, n if act_scale is None else n // 2)
+    d_dtype, kind = (out_kind(d.dtype), 0) if act_scale is None else (out_kind(mid_dtype), fp8_kind(d.dtype))
+    with torch.cuda.device(a.device):
+        return lib.hfrk_wide_gemm_fp8(
+            a.data_ptr(), w.data_ptr(), d.data_ptr(), scale.data_ptr(), 0 if act_scale is None else act_scale.data_ptr(),
+            m, n, k, w.stride(0), fp8_kind(a.dtype), fp8_kind(w.dtype), d_dtype, int(accumulate), kind, split_k, tile_rows,
+            num_stages, ctas_per_sm, _stream_ptr(stream, a.device))
 
 
 MODEL_MAX_SPLIT, MODEL_MAX_PER_SM = 16, 3

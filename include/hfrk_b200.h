@@ -252,8 +252,32 @@ int hfrk_skinny_gemm_fp8_profile(const void* A, const void* W, void* D, const fl
  * out[4]=dynamic shared memory bytes, out[5]=padded token count (MMA N), out[6]=K blocks of 128,
  * out[7]=tiles along N (of out[3]/out[1] CTAs; a tile is at most 128 rows). Describes the kernel that pins
  * apply to, in launches of at most 64 tokens; automatic calls with more tokens (and some from 17 on)
- * run the wide kernel, whose shape follows from (m, n, k) and the device. Returns a status code. */
+ * run the wide kernel: hfrk_gemm_launch_info tells which. Returns a status code. */
 int hfrk_skinny_gemm_plan(int m, int n, int k, int variant, int split_k, int ctas_per_sm, int* out8);
+
+/* The kernel with the tokens on the tensor core's M side, up to 256 of them per launch. Automatic calls
+ * take it by a rule on (m, n, k); it is not a value of enum hfrk_variant. */
+enum { HFRK_KERNEL_WIDE = 3 };
+enum hfrk_gemm_form { HFRK_FORM_ACCUMULATE = 0, HFRK_FORM_STORE = 1, HFRK_FORM_SWIGLU = 2 };
+
+/* The launch a call makes (its first one, where the tokens do not fit in one; no GPU work).
+ *   form   : enum hfrk_gemm_form: hfrk_skinny_gemm_fp8 / _ex on W[n, k] with accumulate = 1 or 0, or
+ *            hfrk_gate_up_swiglu_fp8 with n = 2 * inter
+ *   kernel : enum hfrk_variant as given to _ex with split_k, num_stages and ctas_per_sm (all 0 = the automatic
+ *            call), or HFRK_KERNEL_WIDE = hfrk_wide_gemm_fp8 with the four pins
+ * out[0]=kernel (1 CLUSTER, 2 STREAMK, 3 WIDE), out[1]=split_k (0 for STREAMK), out[2]=num_stages, out[3]=grid
+ * CTAs, out[4]=dynamic shared memory bytes, out[5]=padded token count, out[6]=K blocks of 128, out[7]=W rows per
+ * CTA (swiglu: gate and up rows together). Returns a status code. */
+int hfrk_gemm_launch_info(int m, int n, int k, int form, int kernel, int split_k, int tile_rows, int num_stages,
+                          int ctas_per_sm, int* out8);
+/* The wide kernel with its launch shape pinned (tests, sweeps): D <- [D +] scale * A . W^T, or with act_scale_dev
+ * the swiglu form, D = act_out[m, n / 2] of out_kind, d_dtype the 16-bit type of the projection.
+ *   split_k : 1..8, tile_rows : 32..256 in steps of 16 (swiglu 32), num_stages : at most this many, 2..8,
+ *   ctas_per_sm : 1 or 2 (sets the shared memory of a CTA); 0 = choose each. HFRK_INVALID_CONFIG if no shape
+ *   that the device holds has these values. */
+int hfrk_wide_gemm_fp8(const void* A, const void* W, void* D, const float* scale_dev, const float* act_scale_dev,
+                       int m, int n, int k, int64_t w_row_stride, int a_kind, int w_kind, int d_dtype, int accumulate,
+                       int out_kind, int split_k, int tile_rows, int num_stages, int ctas_per_sm, void* stream);
 
 /* ---- the element-wise kernels either side of the GEMM in a decoder layer -------------------
  * Both quantise the input of the next projection to fp8 and zero the buffer that projection

@@ -195,3 +195,75 @@ def test_fused_swiglu_under_extreme_scales(capi, dev, act, fp8, scale):
     torch.ops._HFRK_C.gate_up_swiglu(a, w.t(), out, s, act_scale, none, act == torch.bfloat16)
     _ok(capi)
     assert torch.equal(out.view(torch.uint8), expect.view(torch.uint8))
+
+
+def _shapes(capi, m, n, k, split, swiglu):
+    """Launch shapes with this K split: one and two CTAs per SM, two stages and as many as fit, of the tile heights
+    that the device holds the lowest, the highest and the ones whose column groups do not divide by the split."""
+    step = 32 if swiglu else 16
+    shapes = []
+    for per_sm in (1, 2):
+        for stages in (2, 0):
+            fits = []
+            for tile in range(32, 257, step):
+                out = (capi.ctypes.c_int * 8)()
+                if capi.lib.hfrk_gemm_launch_info(m, n, k, 2 * swiglu, 3, split, tile, stages, per_sm, out) == 0:
+                    fits.append(tile)
+            uneven = [t for t in fits if t // step % split]
+            shapes += [(per_sm, stages, t) for t in sorted({*fits[:1], *uneven[:1], *uneven[-1:], *fits[-1:]})]
+    return shapes
+
+
+@pytest.mark.parametrize("split", range(1, 9))
+@pytest.mark.parametrize("m", [40, 128, 200])              # one accumulator, all its rows, two
+@pytest.mark.parametrize("n,dtype", [(1000, torch.bfloat16), (1002, torch.float16), (1003, torch.bfloat16), (1003, torch.float32)])
+def test_pinned_launch_shapes_against_float64(capi, dev, m, n, dtype, split):
+    """Rows of D that are 16-byte aligned, 4-byte aligned and neither; accumulating and storing; N that ends
+    inside a tile; eleven K blocks, the last one short, shared out unevenly."""
+    k = 1296
+    a, w, scale = _operands(m, n, k, torch.float8_e4m3fn, dev)
+    d_in = torch.randn((m, n), generator=torch.Generator(device=dev).manual_seed(5), device=dev).to(dtype)
+    prod = (a.double() @ w.double().t()) * scale.double()
+    bound, bound_in = _bound(prod, a, w, scale, dtype), _bound(prod + d_in.double(), a, w, scale, dtype)
+    shapes = _shapes(capi, m, n, k, split, False)
+    assert shapes and (m > 40 or {s[:2] for s in shapes} == {(1, 0), (1, 2), (2, 0), (2, 2)})
+    for per_sm, stages, tile in shapes:
+        backing = torch.full((m * n + 64,), 9.0, dtype=dtype, device=dev)
+        d = backing[32:32 + m * n].view(m, n)
+        pins = dict(split_k=split, tile_rows=tile, num_stages=stages, ctas_per_sm=per_sm)
+        d.copy_(d_in)
+        capi.check(capi.wide_gemm(a, w, d, scale, **pins))
+        _ok(capi)
+        assert bool(((d.double() - prod - d_in.double()).abs() <= bound_in).all()), pins
+        d.fill_(float("nan"))
+        capi.check(capi.wide_gemm(a, w, d, scale, accumulate=False, **pins))
+        _ok(capi)
+        assert bool(((d.double() - prod).abs() <= bound).all()), pins
+        assert bool((backing[:32] == 9).all() and (backing[-32:] == 9).all()), pins
+
+
+@pytest.mark.parametrize("split", range(1, 9))
+@pytest.mark.parametrize("m", [3, 40, 128, 200])
+@pytest.mark.parametrize("act,fp8", [(torch.bfloat16, torch.float8_e4m3fn), (torch.float16, torch.float8_e4m3fnuz)])
+def test_pinned_swiglu_launch_shapes(capi, dev, m, act, fp8, split):
+    """As :func:`test_wide_gate_up_swiglu_against_the_two_launches`, by pinned shapes."""
+    from hf_rocm_kernels import skinny_gemm, swiglu
+
+    inter, k = 528, 1296
+    a, w, scale = _operands(m, 2 * inter, k, fp8, dev)
+    act_scale = torch.tensor([0.02], device=dev)
+    gate_up = torch.zeros((m, 2 * inter), dtype=act, device=dev)
+    skinny_gemm(a, w.t(), scale, gate_up)
+    expect = swiglu(gate_up, act_scale, out_dtype=fp8)
+    shapes = _shapes(capi, m, 2 * inter, k, split, True)
+    assert shapes or (m == 200 and split > 6)     # no room for the partials of so many
+    for per_sm, stages, tile in shapes:
+        pins = dict(split_k=split, tile_rows=tile, num_stages=stages, ctas_per_sm=per_sm)
+        backing = torch.full((m * inter + 64,), 0x55, dtype=torch.uint8, device=dev)
+        out = backing[32:32 + m * inter].view(m, inter).view(fp8)
+        capi.check(capi.wide_gemm(a, w, out, scale, act_scale, mid_dtype=act, **pins))
+        _ok(capi)
+        assert int((out.view(torch.uint8) != expect.view(torch.uint8)).sum()) <= 8 + out.numel() * 2.0 ** -15, pins
+        step = (out.float() - expect.float()).abs()
+        assert bool((step <= expect.float().abs() * 2.0 ** -3 + 2.0 ** -9).all()), pins
+        assert bool((backing[:32] == 0x55).all() and (backing[-32:] == 0x55).all()), pins

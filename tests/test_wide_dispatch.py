@@ -51,7 +51,7 @@ def test_explicit_and_tuned_calls_stay_on_the_kernel_they_name(capi):
 
 @pytest.mark.parametrize("m,kernel", [(1, CLUSTER), (16, CLUSTER), (17, WIDE), (64, WIDE), (65, WIDE), (300, WIDE)])
 def test_swiglu_form(capi, m, kernel):
-    assert capi.launch_info(m, 2048, 1024, swiglu=True)["kernel"] == kernel
+    assert capi.launch_info(m, 2048, 1024, form=2)["kernel"] == kernel
 
 
 @pytest.mark.parametrize("swiglu", [False, True])
@@ -66,7 +66,7 @@ def test_every_pinned_shape_keeps_its_bounds(capi, m, swiglu):
             for stages in (2, 8):
                 for per_sm in (1, 2):
                     out = (capi.ctypes.c_int * 8)()
-                    rc = capi.lib.hfrk_gemm_launch_info(m, 2080, 2064, int(swiglu), WIDE, split, tile, stages, per_sm, out)
+                    rc = capi.lib.hfrk_gemm_launch_info(m, 2080, 2064, 2 * swiglu, WIDE, split, tile, stages, per_sm, out)
                     if rc != 0:
                         assert rc == 6
                         continue
@@ -88,9 +88,10 @@ def test_every_pinned_shape_keeps_its_bounds(capi, m, swiglu):
 
 def test_bad_queries(capi):
     out = (capi.ctypes.c_int * 8)()
-    for args in ((0, 128, 128, 0, 0), (16, 128, 128, 0, 4), (16, 127, 128, 1, 0), (16, 128, 128, 1, 1), (300, 128, 128, 0, -1)):
+    for args in ((0, 128, 128, 0, 0), (16, 128, 128, 0, 4), (16, 127, 128, 2, 0), (16, 128, 128, 2, 1), (16, 128, 128, 3, 0), (300, 128, 128, 0, -1)):
         assert capi.lib.hfrk_gemm_launch_info(*args, 0, 0, 0, 0, out) == 6
     assert capi.lib.hfrk_gemm_launch_info(200, 128, 128, 0, WIDE, 9, 0, 0, 0, out) == 6       # more than eight CTAs per cluster
     assert capi.lib.hfrk_gemm_launch_info(200, 128, 128, 0, WIDE, 2, 0, 0, 0, out) == 6       # more than the K blocks
     assert capi.lib.hfrk_gemm_launch_info(200, 128, 128, 0, WIDE, 0, 40, 0, 0, out) == 6      # no multiple of 16
     assert capi.lib.hfrk_wide_gemm_fp8(0, 0, 0, 0, 0, 16, 128, 128, 128, 0, 0, 1, 0, 0, 0, 0, 0, 0, 0) == 6
+
