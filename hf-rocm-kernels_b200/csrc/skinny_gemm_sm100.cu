@@ -736,19 +736,30 @@ int make_wide_plan(const DeviceModel& dm, int m, int n, int k, bool swiglu, cons
 }
 
 // Which calls the wide kernel takes, unless the caller (or the tuning table) asked for a launch shape of
-// the skinny kernel:
-//   * more tokens than one launch of the skinny kernel holds: 28672 x 4096 at 256 tokens 31 us against 91;
-//   * 17 to 64 tokens where the skinny kernel's unsplit grid needs a second wave, because its activation
-//     tile leaves room for two CTAs per SM: 39840 x 6272 at 30 tokens 42 us against 55;
-//   * 33 to 64 tokens where an owner of its K split finishes more than kOwned token rows and the
-//     reduction runs past its registers, D_in late: 6144 x 4096 at 64 tokens 9.9 us against 12.3,
-//     10240 x 8192 19.2 against 29.1, 8192 x 8192 16.2 against 17.7; overwriting D, the two are even.
-// Elsewhere up to 64 tokens the skinny kernel is ahead (by 1 to 3 us, most at the fewest tokens).
+// the skinny kernel. From 1,076 shapes of 17 to 260 tokens, N of 1,000 to 57,344, K of 512 to 28,672, and 276 of
+// up to 128,256 rows, timed on both kernels, accumulating and storing; the line is drawn by what the skinny
+// kernel's plan would be:
+//   * more tokens than one of its launches holds: always wide (28672 x 4096 at 256 tokens 31 us against 91);
+//   * K split, an owner that finishes up to 8 token rows: skinny (ahead by 5 to 60 %, most at the fewest tokens);
+//     32 rows: wide (14336 x 8192 at 64 tokens 23.9 us against 30.7 accumulating, 24.7 storing);
+//   * 16 rows, accumulating: the skinny reduction runs past its registers and reads D_in late. Wide at 33 to 64
+//     tokens (6144 x 4096 at 64 tokens 9.9 us against 12.3) except on tall tiles with odd N (17435 x 1344 at 41
+//     15.6 against 10.7), and at 17 to 32 (15 % ahead in the middle) except as one long K range per CTA or on
+//     tall tiles with rows of D that are not 16-byte aligned (25 x 17776 x 4672 20.7 us against 19.0; 21 x 18527
+//     x 832 11.9 against 8.6);
+//   * 16 rows, storing: skinny up to 32 tokens (20 x 4384 x 576 5.8 us against 4.3). Above, wide where skinny
+//     CTAs are three to an SM on two stages (39 x 11936 x 8208 21.4 us against 26.4), split two K blocks each
+//     (64 x 8192 x 1024 6.2 against 7.4), or on few tiles with full owners or a long K; not in between
+//     (33 x 10544 x 1568 9.1 against 7.8). What it picks takes 1 % longer than the better kernel on average,
+//     14 % at worst;
+//   * no K split, one wave: skinny. A second wave: wide (39840 x 6272 at 30 tokens 42 us against 55), except
+//     where up to 48 tokens run a long K through waves that are more than two thirds full (57344 x 8192 at 30
+//     tokens 79.7 us against 75.9; 38144 x 8192 52.6 against 65.8).
 bool pins_launch_shape(int variant, int split_req, int ctas_per_sm, int stages_req) {
     return variant != HFRK_VARIANT_AUTO || split_req != 0 || ctas_per_sm != 0 || stages_req != 0;
 }
 
-bool use_wide_kernel(const DeviceModel& dm, int m, int n, int k, bool explicit_shape) {
+bool use_wide_kernel(const DeviceModel& dm, int m, int n, int k, bool accumulate, bool explicit_shape) {
     if (explicit_shape || m <= 16) return false;
     TuneValue tuned;
     const int mc = m < kMaxMPad ? m : kMaxMPad;
@@ -756,7 +767,23 @@ bool use_wide_kernel(const DeviceModel& dm, int m, int n, int k, bool explicit_s
     if (m > kMaxMPad) return true;
     Plan plan;
     if (make_plan(dm, m, n, k, 0, 0, &plan) != HFRK_SUCCESS) return false;
-    return plan.split == 1 ? plan.ctas > ctas_per_sm(plan.smem_bytes) * dm.sms : (1 << plan.rows_log2) > kOwned;
+    if (plan.split == 1) {
+        const int slots = ctas_per_sm(plan.smem_bytes) * dm.sms;
+        const int waves = (plan.ctas + slots - 1) / slots;
+        return waves > 1 && (m > 48 || k <= 3072 || 20ll * waves * slots > 29ll * plan.ctas);
+    }
+    const int rows_per_owner = 1 << plan.rows_log2;
+    if (rows_per_owner != 2 * kOwned) return rows_per_owner > kOwned;
+    if (m > 32 && !accumulate) {
+        return plan.tiles >= 93 || (m > 48 && plan.num_kblocks <= 2 * plan.split) ||
+               (plan.tiles < 70 && (m > 60 || k >= 4400));
+    }
+    WidePlan wide;
+    if (!accumulate || make_wide_plan(dm, m, n, k, false, WideReq(), &wide) != HFRK_SUCCESS) return false;
+    if (wide.split > 1) return true;
+    // D_in is read by the CTA that multiplies: rows of D that are not aligned cost most on tall tiles
+    if (m > 32) return n % 2 == 0 || wide.tile_n <= 64;
+    return wide.num_kblocks <= 13 && (n % 8 == 0 || wide.tile_n <= 64);
 }
 
 int wide_tokens_per_launch(int m) {
@@ -861,7 +888,7 @@ int launch_gemm(const void* A, const void* W, void* D, const float* scale_dev, i
                               ctas_per_sm, stages_req, use_pdl, stream, stamps);
     }
 
-    if (use_wide_kernel(device_model(stream), m, n, k, rowpar != nullptr || explicit_shape)) {
+    if (use_wide_kernel(device_model(stream), m, n, k, accumulate != 0, rowpar != nullptr || explicit_shape)) {
         return launch_wide<false>(A, W, m, n, k, w_row_stride, wide_params(D, scale_dev, a_kind, w_kind, d_dtype, accumulate),
                                   WideReq(), use_pdl, stream);
     }
@@ -1795,7 +1822,8 @@ extern "C" int hfrk_gemm_launch_info(int m, int n, int k, int form, int kernel, 
     bool wide = kernel == HFRK_KERNEL_WIDE;
     if (kernel == HFRK_VARIANT_AUTO) {
         wide = swiglu ? m > 16
-                      : use_wide_kernel(dm, m, n, k, pins_launch_shape(kernel, split_k, ctas_per_sm, num_stages) || tile_rows != 0);
+                      : use_wide_kernel(dm, m, n, k, form == HFRK_FORM_ACCUMULATE,
+                                        pins_launch_shape(kernel, split_k, ctas_per_sm, num_stages) || tile_rows != 0);
     }
     if (wide) {
         WideReq req;

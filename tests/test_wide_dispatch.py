@@ -95,3 +95,36 @@ def test_bad_queries(capi):
     assert capi.lib.hfrk_gemm_launch_info(200, 128, 128, 0, WIDE, 0, 40, 0, 0, out) == 6      # no multiple of 16
     assert capi.lib.hfrk_wide_gemm_fp8(0, 0, 0, 0, 0, 16, 128, 128, 128, 0, 0, 1, 0, 0, 0, 0, 0, 0, 0) == 6
 
+
+ACCUMULATE, STORE = 0, 1
+
+
+# The skinny kernel's plan on the chip above is part of the case: (split, rows per owner) by which the line is drawn.
+@pytest.mark.parametrize("m,n,k,split,rows,accumulate,store", [
+    (24, 4096, 4096, 7, 4, CLUSTER, CLUSTER),        # owners of up to eight rows
+    (48, 6144, 4096, 7, 8, CLUSTER, CLUSTER),
+    (24, 4096, 512, 2, 16, WIDE, CLUSTER),           # sixteen, up to 32 tokens: accumulating calls only
+    (25, 17776, 4672, 2, 16, CLUSTER, CLUSTER),      # ... one long K range per wide CTA
+    (21, 18527, 832, 2, 16, CLUSTER, CLUSTER),       # ... rows of D unaligned, tall tiles
+    (21, 18528, 832, 2, 16, WIDE, CLUSTER),
+    (64, 6144, 4096, 4, 16, WIDE, WIDE),             # 33 to 64 tokens: few tiles, full owners
+    (44, 1288, 992, 4, 16, WIDE, CLUSTER),
+    (33, 10544, 1568, 3, 16, WIDE, CLUSTER),
+    (39, 11936, 8208, 3, 16, WIDE, WIDE),            # 94 tiles
+    (49, 5760, 928, 4, 16, WIDE, WIDE),              # two K blocks per skinny CTA
+    (41, 15435, 1344, 3, 16, CLUSTER, WIDE), (41, 15436, 1344, 3, 16, WIDE, WIDE),   # odd N on tall tiles
+    (64, 14336, 4096, 2, 32, WIDE, WIDE), (54, 8192, 1024, 3, 32, WIDE, WIDE),   # 32 rows per owner
+    (33, 28672, 4096, 1, 0, CLUSTER, CLUSTER),       # no split, one wave
+    (30, 39840, 6272, 1, 0, WIDE, WIDE),             # a second wave that has hardly begun
+    (30, 57344, 8192, 1, 0, CLUSTER, CLUSTER),       # one that is well filled, long K
+    (30, 57344, 2048, 1, 0, WIDE, WIDE),
+    (64, 57344, 8192, 1, 0, WIDE, WIDE),
+])
+def test_17_to_64_tokens(capi, m, n, k, split, rows, accumulate, store):
+    plan = capi.launch_info(m, n, k, kernel=CLUSTER)
+    assert plan["split_k"] == split
+    if split > 1:
+        assert 1 << (-(-m // split) - 1).bit_length() == rows
+    assert capi.launch_info(m, n, k, ACCUMULATE)["kernel"] == accumulate
+    assert capi.launch_info(m, n, k, STORE)["kernel"] == store
+
