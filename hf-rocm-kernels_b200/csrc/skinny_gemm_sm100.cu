@@ -786,6 +786,27 @@ bool use_wide_kernel(const DeviceModel& dm, int m, int n, int k, bool accumulate
     return wide.num_kblocks <= 13 && (n % 8 == 0 || wide.tile_n <= 64);
 }
 
+// Whether the MLP block's gate/up projection runs with swiglu in its epilogue. Up to 16 tokens always (the
+// skinny kernel's own form). Above, that is the wide kernel: one launch of some 3 us less, but a GEMM that is
+// slower than the skinny one where that one splits K into owners of few rows. Measured in chains of MLP blocks
+// (rms, gate/up, swiglu, down) of 1,024 to 8,192 hidden columns and 17 to 64 tokens:
+//   * owners of up to 8 rows: two launches (4096 x 2 * 7168 at 24 tokens 23.7 us a block against 27.5; 2048 x
+//     2 * 4096 13.5 against 17.1; 2192 x 2 * 5584 at 33 19.3 against 20.4), and owners of 16 up to 32 tokens
+//     (8192 x 2 * 7168 at 28 39.1 against 40.3);
+//   * no K split, or owners of 16 and more above 32 tokens: one (4096 x 2 * 14336 at 32 tokens 38.5 us against
+//     40.3, at 64 40.3 against 45.3; 4096 x 2 * 7168 at 40 28.4 against 33.3);
+//   * above 64 tokens one (227 tokens, 4144 x 2 * 9424: 60.5 us against 66.2).
+// A launch shape pinned for the projection is one of two launches.
+bool fuses_swiglu(const DeviceModel& dm, int m, int inter, int k) {
+    if (m <= 16) return true;
+    TuneValue tuned;
+    if (tuning_lookup(round_up(m < kMaxMPad ? m : kMaxMPad, 16), 2 * inter, k, &tuned)) return false;
+    if (m > kMaxMPad) return true;
+    Plan plan;
+    if (make_plan(dm, m, 2 * inter, k, 0, 0, &plan) != HFRK_SUCCESS) return true;
+    return plan.split == 1 || (m > 32 && (1 << plan.rows_log2) > kOwned);
+}
+
 int wide_tokens_per_launch(int m) {
     const int chunks = (m - 1) / kWideMaxTokens + 1;
     return (m - 1) / chunks + 1;
@@ -1368,6 +1389,11 @@ extern "C" int hfrk_gate_up_swiglu_fp8(const void* A, const void* W_gate_up, voi
     return hfrk::launch_gemm_swiglu(A, W_gate_up, act_out, scale_dev, act_scale_dev, next_buffer, m, inter, k,
                                     w_row_stride, a_kind, w_kind, mid_dtype, out_kind, buffer_cols, /*split_req=*/0,
                                     hfrk::default_use_pdl(), /*any_tokens=*/true, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int hfrk_gate_up_fuses(int m, int inter, int k, void* stream) {
+    if (m <= 0 || inter <= 0 || k <= 0 || inter % 16 != 0 || inter > INT32_MAX / 2) return 0;
+    return hfrk::fuses_swiglu(hfrk::device_model(static_cast<cudaStream_t>(stream)), m, inter, k) ? 1 : 0;
 }
 
 extern "C" int hfrk_wide_gemm_fp8(const void* A, const void* W, void* D, const float* scale_dev,

@@ -117,6 +117,22 @@ static void call_gate_up_swiglu(GateUpEntry entry, torch::Tensor& A, torch::Tens
     TORCH_CHECK(status == HFRK_SUCCESS, "skinny_gemm_swiglu: status ", status, " (", hfrk_last_error(), ")");
 }
 
+// hfrk_gate_up_swiglu_fp8 as two launches with the projection in a buffer between them.
+static int gate_up_then_swiglu(const void* A, const void* W, void* act_out, const float* scale_dev,
+                               const float* act_scale_dev, void* next_buffer, int m, int inter, int k,
+                               int64_t w_row_stride, int a_kind, int w_kind, int mid_dtype, int out_kind,
+                               int64_t buffer_cols, void* stream) {
+    if (inter > INT32_MAX / 2) return HFRK_INVALID_CONFIG;
+    const at::Tensor gate_up = at::empty(
+        {m, 2 * static_cast<int64_t>(inter)},
+        at::TensorOptions().device(at::kCUDA).dtype(mid_dtype == HFRK_BF16 ? at::kBFloat16 : at::kHalf));
+    const int status = hfrk_skinny_gemm_fp8(A, W, gate_up.data_ptr(), scale_dev, m, 2 * inter, k, w_row_stride, a_kind, w_kind,
+                                            mid_dtype, /*accumulate=*/0, /*split_k_hint=*/0, stream);
+    if (status != HFRK_SUCCESS) return status;
+    return hfrk_swiglu_fp8(gate_up.data_ptr(), act_scale_dev, act_out, next_buffer, m, inter, buffer_cols, mid_dtype, out_kind,
+                           /*force_scalar=*/0, stream);
+}
+
 // Gate/up projection with swiglu in its epilogue (hfrk_skinny_gemm_fp8_swiglu): A [m, k] fp8, B the
 // [k, 2*inter] view (stride(0) == 1) of the row-major gate/up weight, act_out [m, inter] fp8,
 // next_buffer [m, any] 16-bit zeroed. mid_bf16 names the 16-bit type the unfused chain would have
@@ -126,10 +142,20 @@ void skinny_gemm_swiglu(torch::Tensor& A, torch::Tensor& B, torch::Tensor& act_o
     call_gate_up_swiglu(hfrk_skinny_gemm_fp8_swiglu, A, B, act_out, scale_tensor, act_scale_tensor, next_buffer, mid_bf16);
 }
 
-// The same for any number of tokens (hfrk_gate_up_swiglu_fp8).
+// The same for any number of tokens: one launch (hfrk_gate_up_swiglu_fp8), or above 16 tokens the GEMM and
+// swiglu where those are faster (hfrk_gate_up_fuses) or the buffer is no multiple of 16 bytes.
 void gate_up_swiglu(torch::Tensor& A, torch::Tensor& B, torch::Tensor& act_out, torch::Tensor& scale_tensor,
                     torch::Tensor& act_scale_tensor, torch::Tensor& next_buffer, bool mid_bf16) {
-    call_gate_up_swiglu(hfrk_gate_up_swiglu_fp8, A, B, act_out, scale_tensor, act_scale_tensor, next_buffer, mid_bf16);
+    GateUpEntry entry = hfrk_gate_up_swiglu_fp8;
+    if (A.dim() == 2 && A.size(0) > 16 && A.is_cuda() && B.dim() == 2 && B.size(1) % 32 == 0) {
+        const at::cuda::OptionalCUDAGuard device_guard(device_of(A));
+        const auto clamped = [](int64_t v) { return static_cast<int>(v > INT32_MAX ? INT32_MAX : v); };
+        const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
+        if (next_buffer.numel() % 8 != 0 ||
+            !hfrk_gate_up_fuses(clamped(A.size(0)), clamped(B.size(1) / 2), clamped(A.size(1)), stream))
+            entry = gate_up_then_swiglu;
+    }
+    call_gate_up_swiglu(entry, A, B, act_out, scale_tensor, act_scale_tensor, next_buffer, mid_bf16);
 }
 
 // gate_up [rows, 2*hidden] fp16/bf16 -> output [rows, hidden] fp8 (e4m3fnuz as in the reference, or

@@ -36,7 +36,7 @@ EXPORTED_SYMBOLS = (
     "hfrk_swiglu_fp8", "hfrk_residual_rms", "hfrk_rowpar_set_mode",
     "hfrk_skinny_gemm_fp8_swiglu", "hfrk_gate_up_swiglu_fp8", "hfrk_skinny_gemm_fp8_host_async",
     "hfrk_tuning_set_ex", "hfrk_host_batch_inputs_first", "hfrk_gemm_launch_info",
-    "hfrk_wide_gemm_fp8", "hfrk_rowpar_set_wait_ms", "hfrk_device_model_get", "hfrk_device_model_override",
+    "hfrk_wide_gemm_fp8", "hfrk_gate_up_fuses", "hfrk_rowpar_set_wait_ms", "hfrk_device_model_get", "hfrk_device_model_override",
 )
 
 
@@ -106,6 +106,8 @@ def _load() -> ctypes.CDLL:
     lib.hfrk_gate_up_swiglu_fp8.restype = i32
     lib.hfrk_gemm_launch_info.argtypes = [i32] * 9 + [ctypes.POINTER(i32)]
     lib.hfrk_gemm_launch_info.restype = i32
+    lib.hfrk_gate_up_fuses.argtypes = [i32, i32, i32, vp]
+    lib.hfrk_gate_up_fuses.restype = i32
     lib.hfrk_wide_gemm_fp8.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i64] + [i32] * 9 + [vp]
     lib.hfrk_wide_gemm_fp8.restype = i32
     lib.hfrk_last_error.restype = ctypes.c_char_p

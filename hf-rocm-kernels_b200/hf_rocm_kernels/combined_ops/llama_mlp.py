@@ -58,21 +58,11 @@ def skinny_gemm_swiglu(
     return out
 
 
-def _fuses(tokens: int, hidden: int, intermediate: int) -> bool:
-    """Whether the block folds swiglu into the gate/up projection when the caller does not say. Above 16
-    tokens that is the kernel with the tokens on the tensor core's M side, which starts some 2 us later
-    than the projection alone would: it saves a launch of 3 us, but a small matrix at few tokens gains
-    nothing (20 tokens, 9216 x 1568: four layers 113 us in two launches, 119 us in one; 26 tokens,
-    11168 x 2192: 147 and 145 us)."""
-    if intermediate % 16 != 0:
-        return False
-    return tokens <= 16 or tokens > 32 or 2 * intermediate * hidden >= 20_000_000
-
-
 def _gate_up_swiglu(skinny_a: Tensor, gate_up_weight: Tensor, scale_tensor: Tensor, act_scale_tensor: Tensor,
                     next_buffer: Optional[Tensor], mid_dtype: torch.dtype, out_dtype: torch.dtype) -> Tensor:
-    """:func:`skinny_gemm_swiglu` for any number of tokens. Above 16 tokens it stands in for two launches
-    through ``skinny_gemm`` and ``swiglu`` and refuses what their checks refuse, as they do."""
+    """:func:`skinny_gemm_swiglu` for any number of tokens; above 16 the library takes the faster of one launch
+    and two (``hfrk_gate_up_fuses``). There it stands in for ``skinny_gemm`` and ``swiglu`` and refuses what
+    their checks refuse, as they do."""
     tokens, inter = skinny_a.size(0), gate_up_weight.size(1) // 2
     if tokens > 16:
         skinny_gemm_operand_checks(skinny_a, gate_up_weight, scale_tensor)
@@ -122,8 +112,8 @@ def llama_mlp_combined_ops(
             accepted so that existing callers keep working, not used (the library picks the
             launch shape per (m, n, k), or takes it from its tuning table)
         fuse_swiglu: run the gate/up projection and swiglu as one launch; ``True`` takes the form of
-            :func:`skinny_gemm_swiglu` (at most 16 tokens, the bytes of the two launches), ``None`` one
-            launch for any number of tokens where rows split into 16-byte pieces
+            :func:`skinny_gemm_swiglu` (at most 16 tokens, the bytes of the two launches), ``False``
+            runs the two; ``None`` takes one for up to 16 tokens, and above the faster way for the shape
         down_row_parallel: the exchange object of the ranks that share the block; every rank
             multiplies its slice of the swiglu output by its K shard of the down weight and all
             ranks receive the summed result (same bits on every rank)
@@ -132,7 +122,7 @@ def llama_mlp_combined_ops(
     tokens = attn_output.size(0)
     act_dtype = gate_up_weight.dtype
 
-    hidden, inter = gate_up_weight.size(0), gate_up_weight.size(1) // 2
+    inter = gate_up_weight.size(1) // 2
     # the GEMMs store into fresh buffers; only the row-parallel one adds to what its buffer holds
     mlp_output = torch.empty((tokens, down_weight.size(1)), dtype=attn_output.dtype, device=attn_output.device)
     zeroed = None if down_row_parallel is None else mlp_output
@@ -140,7 +130,7 @@ def llama_mlp_combined_ops(
         input=attn_output, residual=residual, weight=rms_weight, epsilon=rms_epsilon,
         scale_tensor=gate_up_input_scale, next_buffer=None, out_dtype=act_dtype,
     )
-    if fuse_swiglu is None and _fuses(tokens, hidden, inter):
+    if fuse_swiglu is None and inter % 16 == 0:      # the fused form writes rows in 16-byte pieces
         swiglu_out = _gate_up_swiglu(normalized, gate_up_weight, gate_up_output_scale, down_input_scale, zeroed,
                                      attn_output.dtype, down_weight.dtype)
     elif fuse_swiglu:

@@ -353,9 +353,17 @@ int hfrk_gate_up_swiglu_fp8(const void* A, const void* W_gate_up, void* act_out,
                             int m, int inter, int k, int64_t w_row_stride, int a_kind, int w_kind,
                             int mid_dtype, int out_kind, int64_t buffer_cols, void* stream);
 
+/* 1 if hfrk_gate_up_swiglu_fp8 is the faster way to gate/up and swiglu for (m, inter, k) on this device, 0 if
+ * hfrk_skinny_gemm_fp8 (accumulate = 0) and hfrk_swiglu_fp8 are, or a launch shape is pinned for the
+ * projection (no GPU work; `stream` is the one the call will be made on). The torch op gate_up_swiglu follows it. */
+int hfrk_gate_up_fuses(int m, int inter, int k, void* stream);
+
 /* Pins the launch shape of (m, n, k) for every later automatic call in this process: split_k and
  * num_stages as in hfrk_skinny_gemm_fp8_ex (0 = leave that one to the built-in rule; both 0 = drop
- * the entry). Token counts share an entry per multiple of 16. Fed from the JSON the grid search
+ * the entry). Token counts share an entry per multiple of 16, those above 64 that of 64: an entry for 64 tokens
+ * keeps all larger calls on launches of at most 64 tokens, which is slower than the automatic launch of up to
+ * 256 (28672 x 4096 at 256 tokens: 91 us instead of 31). Entries for a gate/up matrix apply to the MLP block
+ * above 16 tokens (gate/up and swiglu then run as two launches) and not to its fused launch up to 16. Fed from the JSON the grid search
  * writes (hf_rocm_kernels/benchmarks/skinny_gemm/grid_search.py); stands where the reference has
  * its hard-coded per-shape table (hf_rocm_kernels/operators/skinny_gemm/wrapped.py:42-102). */
 int hfrk_tuning_set(int m, int n, int k, int split_k, int num_stages);

@@ -267,3 +267,58 @@ def test_pinned_swiglu_launch_shapes(capi, dev, m, act, fp8, split):
         step = (out.float() - expect.float()).abs()
         assert bool((step <= expect.float().abs() * 2.0 ** -3 + 2.0 ** -9).all()), pins
         assert bool((backing[:32] == 0x55).all() and (backing[-32:] == 0x55).all()), pins
+
+
+# (24, 9488, 256): one launch without a K split; (40, 1040, 1024) with one; (24, 1040, 1024), (48, 3584, 4096): two
+@pytest.mark.parametrize("m,inter,k,fuses", [(24, 9488, 256, 1), (40, 1040, 1024, 1), (24, 1040, 1024, 0), (48, 3584, 4096, 0)])
+@pytest.mark.parametrize("act,fp8", [(torch.bfloat16, torch.float8_e4m3fn), (torch.float16, torch.float8_e4m3fnuz)])
+def test_gate_up_op_runs_what_the_rule_names(capi, dev, m, inter, k, fuses, act, fp8):
+    """The bytes of the op are those of the one launch or of the two, also with a launch shape pinned for the
+    projection and with a buffer that is no multiple of 16 bytes (two launches in both cases)."""
+    from hf_rocm_kernels import swiglu
+
+    a, w, scale = _operands(m, 2 * inter, k, fp8, dev)
+    act_scale = torch.tensor([0.02], device=dev)
+
+    def op(cols):
+        out, buffer = torch.empty((m, inter), dtype=fp8, device=dev), torch.ones((m, cols), dtype=act, device=dev)
+        torch.ops._HFRK_C.gate_up_swiglu(a, w.t(), out, scale, act_scale, buffer, act == torch.bfloat16)
+        _ok(capi)
+        assert int(buffer.count_nonzero()) == 0
+        return out.view(torch.uint8)
+
+    def two_launches():
+        gate_up = torch.empty((m, 2 * inter), dtype=act, device=dev)
+        torch.ops._HFRK_C.skinny_gemm_store(a, w.t(), gate_up, scale)
+        return swiglu(gate_up, act_scale, out_dtype=fp8).view(torch.uint8)
+
+    one = torch.empty((m, inter), dtype=fp8, device=dev)
+    capi.check(capi.wide_gemm(a, w, one, scale, act_scale, mid_dtype=act))
+    with torch.cuda.device(dev):
+        assert capi.lib.hfrk_gate_up_fuses(m, inter, k, 0) == fuses
+    assert torch.equal(op(8), one.view(torch.uint8) if fuses else two_launches())
+    assert torch.equal(op(5), two_launches() if m * 5 % 8 else op(8))
+    capi.lib.hfrk_tuning_set(m, 2 * inter, k, 2, 2)
+    try:
+        assert torch.equal(op(8), two_launches())
+    finally:
+        capi.lib.hfrk_tuning_clear()
+
+
+@pytest.mark.parametrize("tokens,hidden,inter", [(24, 256, 9488), (40, 1024, 1040)])
+def test_mlp_block_takes_swiglu_in(capi, dev, tokens, hidden, inter):
+    """The block's automatic form above 16 tokens, on shapes where that is one launch, against the two."""
+    from hf_rocm_kernels.combined_ops import llama_mlp_combined_ops
+
+    assert capi.lib.hfrk_gate_up_fuses(tokens, inter, hidden, 0) == 1
+    gen = torch.Generator(device=dev).manual_seed(3)
+    attn, residual = (torch.randn((tokens, hidden), generator=gen, device=dev).to(torch.bfloat16) for _ in range(2))
+    _, w_gu, s_gu = _operands(1, 2 * inter, hidden, torch.float8_e4m3fn, dev)
+    _, w_dn, s_dn = _operands(2, hidden, inter, torch.float8_e4m3fn, dev)
+    act_scale, norm = torch.tensor([0.02], device=dev), torch.ones(hidden, dtype=torch.bfloat16, device=dev)
+    outs = [llama_mlp_combined_ops(attn, residual.clone(), norm, 1e-5, w_gu.t(), act_scale, s_gu * 0.02, w_dn.t(), act_scale,
+                                   s_dn * 0.02, **kw) for kw in ({}, {"fuse_swiglu": False})]
+    _ok(capi)
+    assert torch.equal(outs[0][1], outs[1][1])
+    error = (outs[0][0].double() - outs[1][0].double()).norm() / outs[1][0].double().norm()
+    assert float(error) <= 2.0 ** -9                       # a few outputs one bf16 step (2^-8) apart at most

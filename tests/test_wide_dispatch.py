@@ -128,3 +128,24 @@ def test_17_to_64_tokens(capi, m, n, k, split, rows, accumulate, store):
     assert capi.launch_info(m, n, k, ACCUMULATE)["kernel"] == accumulate
     assert capi.launch_info(m, n, k, STORE)["kernel"] == store
 
+
+@pytest.mark.parametrize("m,inter,k,fuses", [
+    (1, 1040, 1024, 1), (16, 14336, 4096, 1),        # up to 16 tokens always
+    (17, 1040, 1024, 0), (24, 7168, 4096, 0),        # owners of up to eight rows
+    (28, 7168, 8192, 0),                             # sixteen, up to 32 tokens
+    (40, 1040, 1024, 1), (40, 7168, 4096, 1), (48, 3584, 4096, 0), (64, 3584, 4096, 1),
+    (17, 14336, 4096, 1), (24, 9488, 256, 1),        # no K split
+    (65, 1040, 1024, 1), (1000, 14336, 4096, 1), (17, 1032, 1024, 0), (0, 1040, 1024, 0)])
+def test_where_gate_up_takes_swiglu_in(capi, m, inter, k, fuses):
+    assert capi.lib.hfrk_gate_up_fuses(m, inter, k, 0) == fuses
+
+
+def test_a_pinned_projection_is_a_launch_of_its_own_above_16_tokens(capi):
+    for m, bucket in ((16, 16), (40, 48), (64, 64), (200, 64)):
+        assert capi.lib.hfrk_gate_up_fuses(m, 1040, 1024, 0) == 1
+        capi.lib.hfrk_tuning_set(bucket, 2080, 1024, 2, 3)
+        try:
+            assert capi.lib.hfrk_gate_up_fuses(m, 1040, 1024, 0) == int(m <= 16)
+            assert capi.lib.hfrk_gate_up_fuses(m, 1056, 1024, 0) == 1
+        finally:
+            capi.lib.hfrk_tuning_clear()
