@@ -667,7 +667,7 @@ int search_wide_plan(const DeviceModel& dm, int m, int n, int k, bool swiglu, co
             if (req.tile_n != 0 && tile_n != req.tile_n) continue;
             const int groups = tile_n / step;
             if (groups < split) continue;   // every CTA of a cluster finishes something
-            const int tiles = (n + tile_n - 1) / tile_n;
+            const int tiles = (n - 1) / tile_n + 1;
             int acc_cols = 32;
             while (acc_cols < tile_n) acc_cols *= 2;
             const int tmem_cols = halves * acc_cols;
@@ -735,6 +735,12 @@ int make_wide_plan(const DeviceModel& dm, int m, int n, int k, bool swiglu, cons
     return rc;
 }
 
+constexpr int kWideMaxRows = INT32_MAX - kWideMaxTile;   // columns of a tile that ends past N are counted in 32 bits
+
+bool pins_launch_shape(int variant, int split_req, int ctas_per_sm, int stages_req) {
+    return variant != HFRK_VARIANT_AUTO || split_req != 0 || ctas_per_sm != 0 || stages_req != 0;
+}
+
 // Which calls the wide kernel takes, unless the caller (or the tuning table) asked for a launch shape of
 // the skinny kernel. From 1,076 shapes of 17 to 260 tokens, N of 1,000 to 57,344, K of 512 to 28,672, and 276 of
 // up to 128,256 rows, timed on both kernels, accumulating and storing; the line is drawn by what the skinny
@@ -755,15 +761,12 @@ int make_wide_plan(const DeviceModel& dm, int m, int n, int k, bool swiglu, cons
 //   * no K split, one wave: skinny. A second wave: wide (39840 x 6272 at 30 tokens 42 us against 55), except
 //     where up to 48 tokens run a long K through waves that are more than two thirds full (57344 x 8192 at 30
 //     tokens 79.7 us against 75.9; 38144 x 8192 52.6 against 65.8).
-bool pins_launch_shape(int variant, int split_req, int ctas_per_sm, int stages_req) {
-    return variant != HFRK_VARIANT_AUTO || split_req != 0 || ctas_per_sm != 0 || stages_req != 0;
-}
-
 bool use_wide_kernel(const DeviceModel& dm, int m, int n, int k, bool accumulate, bool explicit_shape) {
     if (explicit_shape || m <= 16) return false;
     TuneValue tuned;
     const int mc = m < kMaxMPad ? m : kMaxMPad;
     if (tuning_lookup(round_up(mc, 16), n, k, &tuned)) return false;
+    if (n > kWideMaxRows) return false;
     if (m > kMaxMPad) return true;
     Plan plan;
     if (make_plan(dm, m, n, k, 0, 0, &plan) != HFRK_SUCCESS) return false;
@@ -1414,6 +1417,7 @@ extern "C" int hfrk_wide_gemm_fp8(const void* A, const void* W, void* D, const f
                                   d_dtype, out_kind, /*buffer_cols=*/0, /*split_req=*/0, default_use_pdl(),
                                   /*any_tokens=*/true, s, &req);
     }
+    if (n > kWideMaxRows) return HFRK_INVALID_CONFIG;
     int rc = validate(A, W, D, scale_dev, m, n, k, w_row_stride, a_kind, w_kind, d_dtype);
     if (rc != HFRK_SUCCESS) return rc;
     rc = prepare_device_once();

@@ -149,3 +149,11 @@ def test_a_pinned_projection_is_a_launch_of_its_own_above_16_tokens(capi):
             assert capi.lib.hfrk_gate_up_fuses(m, 1056, 1024, 0) == 1
         finally:
             capi.lib.hfrk_tuning_clear()
+
+
+@pytest.mark.parametrize("m", [17, 65])
+def test_rows_that_a_32_bit_column_cannot_count_stay_on_the_skinny_kernel(capi, m):
+    """The last wide tile would end past 2^31 and write in front of its row."""
+    assert capi.launch_info(m, 2 ** 31 - 200, 16)["kernel"] == CLUSTER
+    assert capi.launch_info(m, 2 ** 31 - 300, 16)["kernel"] == WIDE
+    assert capi.lib.hfrk_wide_gemm_fp8(16, 16, 16, 16, 0, m, 2 ** 31 - 200, 16, 16, 0, 0, 1, 0, 0, 0, 0, 0, 0, 0) == 6
