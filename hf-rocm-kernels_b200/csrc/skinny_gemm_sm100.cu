@@ -312,7 +312,7 @@ int make_plan(const DeviceModel& dm, int m, int n, int k, int split_req, int sta
                 // whose longest range is two as well only adds partials (1400 x 2256: 3.4 us with 9, 3.7 with 13).
                 for (int s = kMaxSplit; s >= 2; --s) {
                     if (nkb / s < 2) {
-                        const bool few = m_pad == 16 && s <= nkb && tiles * s <= dm.sms;
+                        const bool few = m_pad == 16 && s <= nkb && tiles * s <= dm.sms && (nkb > 2 || n % 16 != 0);
                         const bool same_range = s < nkb && nkb % 2 == 0 && nkb / 2 <= kMaxSplit &&
                                                 resident(nkb / 2, ring, spare_clusters(nkb / 2));
                         if (!few || same_range) continue;

@@ -68,8 +68,9 @@ def test_how_many_clusters_stay_free(capi, m, tiles, k, split, smaller, two):
 @pytest.mark.parametrize("n,k,split", [
     (1104, 1104, 9), (848, 2032, 16),               # one K block per CTA
     (848, 2368, 16), (1808, 1808, 9),               # one or two, where half as many CTAs would have up to three
+    (2416, 256, 1), (2360, 256, 2),                 # two in all, whole pieces of 16 rows and not
     (1400, 2256, 9), (1696, 1536, 6), (704, 4096, 16), (648, 3040, 12)])   # two each: no more CTAs for the same longest range
 def test_more_ctas_only_for_a_shorter_range(capi, n, k, split):
     assert _plan(capi, 16, n, k, {})["split_k"] == split
-    if -(-k // 128) % split == 0 and -(-k // 128) // split == 2:      # the split of two each does not fit: then more
+    if split > 1 and -(-k // 128) % split == 0 and -(-k // 128) // split == 2:      # the split of two each does not fit: then more
         assert _plan(capi, 16, n, k, {split: 1})["split_k"] != split
