@@ -135,7 +135,7 @@ swiglu_fp8_vec8_kernel(const T* __restrict__ gate_up, const float* __restrict__ 
         dst[to2] = swiglu_8<T, kFnuz>(g2, u2, inv_scale);
         advance();
     }
-    zero_range(next_buffer, buffer_bytes);
+    zero_range_shared(next_buffer, buffer_bytes);
 }
 
 // Scalar path: any hidden, any alignment.

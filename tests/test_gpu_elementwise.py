@@ -472,3 +472,25 @@ def test_llama_mlp_chain_equals_its_parts_and_tracks_the_unquantised_block(capi,
     expect = (torch.nn.functional.silu(gu[:, :inter]) * gu[:, inter:]) @ p["w_dn"].t()
     error = (out.float() - expect).norm() / expect.norm()
     assert float(error) < 0.15, float(error)      # fp8 on both operands of both GEMMs: ~5 % each
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1024), (1, 1001), (300, 256), (40, 2000)])     # one CTA and many, both kernels
+@pytest.mark.parametrize("offset", [0, 1, 5, 7])                                        # 2-byte elements before the buffer
+@pytest.mark.parametrize("per_row", [1, 3, 8, 1000, 4099])
+def test_every_element_of_the_buffer_is_zeroed_and_no_other(capi, dev, rows, cols, offset, per_row):
+    """Buffers from one element to more pieces than threads, at every kind of alignment, by both kernels."""
+    gate_up = torch.randn((rows, 2 * cols), device=dev).to(torch.bfloat16)
+    scale = torch.tensor([0.05], device=dev)
+    size = rows * per_row
+    for kernel in ("swiglu", "residual_rms"):
+        backing = torch.full((offset + size + 24,), 3.0, dtype=torch.bfloat16, device=dev)
+        buffer = backing[offset + 8:offset + 8 + size].view(rows, per_row)
+        out = torch.empty((rows, cols), dtype=torch.float8_e4m3fn, device=dev)
+        if kernel == "swiglu":
+            capi.check(capi.swiglu(gate_up, scale, out, buffer))
+        else:
+            x, res = gate_up[:, :cols].contiguous(), gate_up[:, cols:].contiguous()
+            capi.check(capi.residual_rms(x, res, torch.ones(cols, dtype=torch.bfloat16, device=dev), scale, 1e-5, out, buffer))
+        torch.cuda.synchronize()
+        assert int(buffer.count_nonzero()) == 0
+        assert bool((backing[:offset + 8] == 3).all() and (backing[offset + 8 + size:] == 3).all())
