@@ -518,6 +518,11 @@ int scratch_for(cudaStream_t stream, float** partials, unsigned int** counters) 
     return HFRK_SUCCESS;
 }
 
+// CTAs that share an SM must never ask for more TMEM than it has: a CTA that waits for columns keeps its
+// cluster waiting. Every kernel's share of the shared memory is at least its share of the 512 columns, so
+// what fits in shared memory fits in TMEM (the cluster kernel's two smallest stages are more than its 32 or 64 columns).
+int tmem_smem_floor(int columns) { return kSmemPerSm / 512 * columns - kSmemCtaReserve; }
+
 struct SkPlan {
     int grid, stages, units_per_stage, smem_bytes, m_pad, nkb, tiles;
 };
@@ -550,6 +555,8 @@ int make_sk_plan(int m, int n, int k, int ctas_per_sm, int stages_req, SkPlan* p
     plan->stages = stages;
     plan->units_per_stage = ups;
     plan->smem_bytes = 1024 + stages * stage_bytes + kCtrlBytes;
+    const int smem_floor = tmem_smem_floor(m_pad <= 16 ? 32 : m_pad <= 32 ? 64 : 128);   // two stages ask for less
+    if (plan->smem_bytes < smem_floor) plan->smem_bytes = smem_floor;
     plan->m_pad = m_pad;
     plan->nkb = nkb;
     plan->tiles = tiles;
@@ -685,10 +692,7 @@ int search_wide_plan(const DeviceModel& dm, int m, int n, int k, bool swiglu, co
                 if (recv_bytes > stages * stage_bytes) continue;
                 if (split > 1 && tiles > dm.capacity[split][per_sm]) continue;
                 int smem = 1024 + stages * stage_bytes + kCtrlBytes;
-                // CTAs that share an SM must never ask for more TMEM than it has: a CTA that waits for
-                // columns keeps its cluster waiting. Every kernel's share of the shared memory is at least its
-                // share of the 512 columns, so what fits in shared memory fits in TMEM.
-                const int smem_floor = kSmemPerSm / 512 * tmem_cols - kSmemCtaReserve;
+                const int smem_floor = tmem_smem_floor(tmem_cols);
                 if (smem < smem_floor) smem = smem_floor;
                 if (smem > kSmemLimit) continue;
 

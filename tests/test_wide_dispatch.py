@@ -157,3 +157,15 @@ def test_rows_that_a_32_bit_column_cannot_count_stay_on_the_skinny_kernel(capi, 
     assert capi.launch_info(m, 2 ** 31 - 200, 16)["kernel"] == CLUSTER
     assert capi.launch_info(m, 2 ** 31 - 300, 16)["kernel"] == WIDE
     assert capi.lib.hfrk_wide_gemm_fp8(16, 16, 16, 16, 0, m, 2 ** 31 - 200, 16, 16, 0, 0, 1, 0, 0, 0, 0, 0, 0, 0) == 6
+
+
+@pytest.mark.parametrize("kernel", [CLUSTER, STREAMK])
+@pytest.mark.parametrize("m,columns", [(1, 32), (16, 32), (17, 64), (32, 64), (33, 128), (48, 128), (64, 128)])
+def test_shared_memory_covers_the_tmem_columns(capi, kernel, m, columns):
+    """CTAs of any two kernels that fit on an SM by shared memory fit by TMEM columns (512) too."""
+    if kernel == CLUSTER:
+        columns = 32 if m <= 32 else 64
+    for stages in (2, 3, 8):
+        for split in ((1, 4) if kernel == CLUSTER else (0,)):
+            info = capi.launch_info(m, 8192, 8192, kernel=kernel, num_stages=stages, split_k=split)
+            assert info["num_stages"] == stages and (info["smem_bytes"] + 1024) * 512 >= columns * 228 * 1024
