@@ -229,7 +229,7 @@ constexpr BuiltinShape kBuiltinShapes[] = {
 //   * three CTAs per SM (a ring of three 18 KiB stages) beat two (four stages) on most shapes:
 //     the third slot lets part of the NEXT call's grid move in and start its weight stream while
 //     this call drains;
-//   * at least two K blocks per CTA once the CTAs outnumber the SMs; no split once the tiles alone cover the SMs (then six
+//   * at least two K blocks per CTA once the CTAs outnumber the SMs, fewer before that only for a shorter longest range; no split once the tiles alone cover the SMs (then six
 //     stages, two CTAs per SM, or three stages when that saves a wave: 448 tiles on 444 slots);
 //   * tiles of fewer than 128 rows even out a grid without a K split that is between one and two
 //     CTAs per SM: 224 tiles of 128 rows put two CTAs on 76 SMs and one on the other 72; 256
@@ -634,10 +634,10 @@ struct WideReq {
     int split = 0, tile_n = 0, stages = 0, per_sm = 0;   // 0 = choose
 };
 
-// Estimated time of one launch in microseconds. The stream of K blocks runs at the slowest of: W out of
+// Estimated time of one launch in microseconds, for choosing among launch shapes of this kernel alone. The stream of K blocks runs at the slowest of: W out of
 // HBM, all loads out of L2, the loads of the busiest SM, the tensor core of the busiest SM, and the
 // latency of a load over the stages that hide it. To it come the fixed cost of a call in a chain of
-// dependent calls, one per further wave, the epilogue's stores and, with a K split, the cluster barrier
+// dependent calls, one per further wave, the epilogue (of which the fit left next to nothing) and, with a K split, the cluster barrier
 // and the partials that a CTA sends to its peers (~40 GB/s per SM). The constants are a fit to
 // 10,400 timings on a B200 (148 shapes of 17 to 256 tokens, every tile height, split and CTAs per SM that
 // fits): the shape it picks is on average 4.5 % slower than the best of its list, 26 % at worst.

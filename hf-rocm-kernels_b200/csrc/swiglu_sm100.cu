@@ -10,12 +10,13 @@
 //
 // HBM should bound it (4 bytes read and 1 written per output element), but at 31 instructions per
 // element the issue slots did: 41.2 us at 2048 x 14336 (3.56 TB/s, 75 % of the issue slots busy, DRAM 39 %).
-// Now 23 per element: two fp32 operations per instruction and a cheaper correctly rounded quotient
-// (silu_f32x2), row and column carried along instead of two 64-bit divisions per vector, and the scale
-// of e4m3fnuz folded into the factor: 27.7 us (5.3 TB/s; what is left is mostly expf and the conversions).
+// Now 23 per element: two fp32 operations per instruction and a cheaper quotient with the same bits for every
+// 16-bit gate (silu_f32x2), row and column carried along instead of two 64-bit divisions per vector, and the scale
+// of e4m3fnuz folded into the factor: 29 to 31 us (4.7 to 5.1 TB/s, issue slots 70 % busy; what is left is mostly
+// expf and the conversions).
 // Every thread owns 8 consecutive outputs of one row (two 16-byte loads, one 8-byte store), two such
 // vectors in flight. CTAs of 128 threads, at most 16 per SM, stride over the matrix: ten of them are
-// resident, the others even out the end (300 x 14336: 6.0 us, 7.2 us as CTAs of 256 that each do their
+// resident, the others even out the end (300 x 14336: 6.2 us, 7.2 us as CTAs of 256 that each do their
 // two vectors and leave, 6.3 us with just the CTAs that are resident), so
 // rows of any length keep all SMs loading. It is launched as a
 // programmatic dependent of the GEMM before it and releases the GEMM after it at once: that

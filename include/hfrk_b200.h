@@ -55,10 +55,11 @@ enum hfrk_fp8_kind { HFRK_E4M3FN = 0, HFRK_E4M3FNUZ = 1 };
 /* F32 output exists for unfused multi-GPU baselines (partial sums that a library all-reduce adds). */
 enum hfrk_out_dtype { HFRK_F16 = 0, HFRK_BF16 = 1, HFRK_F32 = 2 };
 
-/* The two kernels behind the GEMM.
+/* The two kernels behind the GEMM that a call can name (calls above 64 tokens, and some from 17 on, run a third one
+ * automatically: HFRK_KERNEL_WIDE below).
  *   CLUSTER : one CTA per (128-row tile, K split); the K splits of a tile form a thread-block
  *             cluster and reduce through distributed shared memory. No scratch memory.
- *             This is what AUTO picks.
+ *             This is what AUTO picks up to 16 tokens, and above where it is the faster one.
  *   STREAMK : the (tile, K block) work items are cut into equal ranges over a grid sized to the
  *             SM count; partial tiles meet in library-owned fp32 scratch and the last CTA to
  *             arrive reduces them in a fixed order. Balanced for any shape, but its reduction
@@ -66,7 +67,7 @@ enum hfrk_out_dtype { HFRK_F16 = 0, HFRK_BF16 = 1, HFRK_F32 = 2 };
 enum hfrk_variant { HFRK_VARIANT_AUTO = 0, HFRK_VARIANT_CLUSTER = 1, HFRK_VARIANT_STREAMK = 2 };
 
 /* Single-GPU skinny GEMM on `stream` (a cudaStream_t passed as void*), asynchronous, no host
- * synchronisation. The kernel this entry point launches (the cluster kernel) needs no scratch and
+ * synchronisation. The kernels this entry point launches (cluster and wide) need no scratch and
  * the call allocates no device memory; the first call on a device sets the kernels' attributes,
  * so make one call per device before capturing into a CUDA graph. Only the stream-K variant
  * (hfrk_skinny_gemm_fp8_ex with HFRK_VARIANT_STREAMK) owns scratch: about 80 MB per device,
