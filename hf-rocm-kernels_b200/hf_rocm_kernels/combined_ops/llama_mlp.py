@@ -21,8 +21,7 @@ from torch import Tensor
 import hf_rocm_kernels._HFRK_C  # noqa: F401  (registers torch.ops._HFRK_C)
 from hf_rocm_kernels import residual_rms, swiglu
 from hf_rocm_kernels.combined_ops.row_parallel import RowParallelSkinnyGemm
-from hf_rocm_kernels.operators.skinny_gemm.wrapped import (skinny_gemm_checks, skinny_gemm_into_empty,
-                                                           skinny_gemm_operand_checks)
+from hf_rocm_kernels.operators.skinny_gemm.wrapped import skinny_gemm_checks, skinny_gemm_into_empty
 
 
 def can_fuse_swiglu(tokens: int, hidden: int, intermediate: int) -> bool:
@@ -65,7 +64,7 @@ def _gate_up_swiglu(skinny_a: Tensor, gate_up_weight: Tensor, scale_tensor: Tens
     their checks refuse, as they do."""
     tokens, inter = skinny_a.size(0), gate_up_weight.size(1) // 2
     if tokens > 16:
-        skinny_gemm_operand_checks(skinny_a, gate_up_weight, scale_tensor)
+        skinny_gemm_checks(skinny_a, gate_up_weight, scale_tensor, None)
         assert gate_up_weight.size(1) % 2 == 0, f"Expected an even number of columns: {gate_up_weight.shape = }."
         assert act_scale_tensor.numel() == 1, f"Expected {act_scale_tensor.numel() = } to be 1."
         assert act_scale_tensor.device == skinny_a.device, \

@@ -33,10 +33,17 @@ _STATUS_TEXT = {
 }
 
 
-def skinny_gemm_operand_checks(skinny_a: Tensor, b: Tensor, scale_tensor: Tensor) -> None:
-    """Raises AssertionError unless the inputs form a valid call (shapes, layouts, dtypes, device)."""
+def skinny_gemm_checks(
+    skinny_a: Tensor,
+    b: Tensor,
+    scale_tensor: Tensor,
+    output: Optional[Tensor],
+) -> None:
+    """Raises AssertionError unless the four tensors form a valid call (shapes, layouts, dtypes, device).
+    ``output`` is ``None`` for a launch that does not write the product itself."""
+    m, k = skinny_a.size(0), skinny_a.size(1)
     assert skinny_a.dim() == 2, f"Expected skinny_a to have 2 dimensions but got {skinny_a.dim() = } instead."
-    assert b.dim() == 2 and skinny_a.size(1) == b.size(0), f"Expected {skinny_a.size(1) = } and {b.size(0) = } to be the same."
+    assert b.dim() == 2 and k == b.size(0), f"Expected {skinny_a.size(1) = } and {b.size(0) = } to be the same."
     assert scale_tensor.numel() == 1, f"Expected {scale_tensor.numel() = } to be 1."
     assert skinny_a.is_contiguous(), f"Expected skinny_a to be contiguous but got {skinny_a.stride() = }"
     assert b.stride(0) == 1, f"Expected b to be column-major but got {b.stride() = }"
@@ -47,22 +54,13 @@ def skinny_gemm_operand_checks(skinny_a: Tensor, b: Tensor, scale_tensor: Tensor
     assert device.type == "cuda", f"Expected input.device to be of type cuda, but got {device.type = } instead."
     for name, tensor in (("b", b), ("scale_tensor", scale_tensor)):
         assert tensor.device == device, f"Expected {name}.device = {tensor.device} to be the same as {device = }"
-
-
-def skinny_gemm_checks(
-    skinny_a: Tensor,
-    b: Tensor,
-    scale_tensor: Tensor,
-    output: Tensor,
-) -> None:
-    """Raises AssertionError unless the four tensors form a valid call (shapes, layouts, dtypes, device)."""
-    skinny_gemm_operand_checks(skinny_a, b, scale_tensor)
-    assert tuple(output.shape) == (skinny_a.size(0), b.size(1)), (
+    if output is None:
+        return
+    assert tuple(output.shape) == (m, b.size(1)), (
         f"{tuple(output.shape)} does not match with {tuple(skinny_a.shape) = } and {tuple(b.shape) = }")
     assert output.is_contiguous(), f"Expected output to be contiguous but got {output.stride() = }"
     assert output.dtype in _OUT_DTYPES, f"Expected {output.dtype = } to be one of {_OUT_DTYPES}"
-    assert output.device == skinny_a.device, \
-        f"Expected output.device = {output.device} to be the same as {skinny_a.device = }"
+    assert output.device == device, f"Expected output.device = {output.device} to be the same as {device = }"
 
 
 def infer_skinny_gemm_params(skinny_a: Tensor, b: Tensor) -> Dict[str, int]:
