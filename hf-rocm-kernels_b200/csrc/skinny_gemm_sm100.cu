@@ -310,12 +310,16 @@ int make_plan(const DeviceModel& dm, int m, int n, int k, int split_req, int sta
                 // 3.4 us with clusters of 4, 2.9 with clusters of 9), and so are one or two, where the split that
                 // gives every CTA two has a CTA with three (848 x 2368: 3.4 us with 9, 3.2 with 16). A larger split
                 // whose longest range is two as well only adds partials (1400 x 2256: 3.4 us with 9, 3.7 with 13).
+                int two_each = -1;   // whether nkb / 2 CTAs of two K blocks fit; asked once, as plans are made on every call
                 for (int s = kMaxSplit; s >= 2; --s) {
                     if (nkb / s < 2) {
                         const bool few = m_pad == 16 && s <= nkb && tiles * s <= dm.sms && (nkb > 2 || n % 16 != 0);
-                        const bool same_range = s < nkb && nkb % 2 == 0 && nkb / 2 <= kMaxSplit &&
-                                                resident(nkb / 2, ring, spare_clusters(nkb / 2));
-                        if (!few || same_range) continue;
+                        if (!few) continue;
+                        if (s < nkb) {
+                            if (two_each < 0)
+                                two_each = nkb % 2 == 0 && nkb / 2 <= kMaxSplit && resident(nkb / 2, ring, spare_clusters(nkb / 2));
+                            if (two_each) continue;
+                        }
                     }
                     if (!resident(s, ring, spare_clusters(s))) continue;
                     const int ctas = tiles * s;
