@@ -367,7 +367,7 @@ __device__ __forceinline__ void wide_epilogue_owner(const WideParams& p, const f
     const int lo = wide_first_group(rank, groups, p.split), own = wide_first_group(rank + 1, groups, p.split) - lo;
     const int rows = p.halves * p.rows_half, pieces = 2 * own > 0 ? 2 * own : 1, items = own > 0 ? rows * pieces : 0;
     const int n0 = blockIdx.x * p.tile_n + lo * 16;
-    Raw8<DT> din[kAhead];
+    Raw8<DT> din[kAhead] = {};
     auto load_ahead = [&](int base) {
 #pragma unroll
         for (int i = 0; i < kAhead; ++i) {
@@ -376,7 +376,7 @@ __device__ __forceinline__ void wide_epilogue_owner(const WideParams& p, const f
             din[i] = wide_load_din<DT>(p, row, n0 + (item - row * pieces) * 8, item < items);
         }
     };
-    load_ahead(threadIdx.x);
+    if (p.accumulate) load_ahead(threadIdx.x);
     const bool ok = wait_accum();
     send();
     if (own == 0) return;
@@ -384,7 +384,7 @@ __device__ __forceinline__ void wide_epilogue_owner(const WideParams& p, const f
     const bool landed = mbar_wait_bounded(recv_bar, 0u, &own_abort, kRoleEpilogue);
     if (!landed || !ok) return;
     for (int base = threadIdx.x; base < items; base += kAhead * kStep) {
-        if (base != static_cast<int>(threadIdx.x)) load_ahead(base);
+        if (p.accumulate && base != static_cast<int>(threadIdx.x)) load_ahead(base);
 #pragma unroll
         for (int i = 0; i < kAhead; ++i) {
             const int item = base + i * kStep;
